@@ -204,9 +204,13 @@ def prepare(case, seed):
     if kind == "sweep":
         ws = _sweep(case, seed)
         batch = pearl_gpu.Batch([(p, c.shape[1], c.shape[0]) for p, _, _, c, _ in ws])
+        # all instances' frames in three buffers, one after another
+        ends = np.cumsum([0] + [c.size for _, _, _, c, _ in ws])
+        flat = [_pinned(k * int(ends[-1])) for k in (3, 1, 1)]
+        out = [tuple(f[k * a:k * b].reshape(w[2 + j].shape) for j, (f, k) in enumerate(zip(flat, (3, 1, 1))))
+               for w, a, b in zip(ws, ends[:-1], ends[1:])]
         return dict(case=case, batch=batch, host=[tuple(map(_pin, f)) for _, _, *f in ws],
-                    scalars=[_scalars(c, dt) for _, dt, _, c, _ in ws],
-                    out=[(_pinned(*phi.shape), _pinned(*c.shape), _pinned(*c.shape)) for _, _, phi, c, _ in ws])
+                    scalars=[_scalars(c, dt) for _, dt, _, c, _ in ws], flat=flat, out=out)
     nx, ny = case["nx"], case["ny"]
     if kind == "init":
         prm = _params(nx, ny, case["cooling"], 4e-12, 4e-12)
@@ -258,7 +262,7 @@ def run(state):
         if any(status):
             raise RuntimeError("an instance failed")
         end = [batch.download(i, out)[3] for i, out in enumerate(state["out"])]
-        flat = [np.concatenate([o[k].reshape(-1) for o in state["out"]]) for k in range(3)]
+        flat = state["flat"]
         return dict(phi=flat[0], carbon=flat[1], mu=flat[2], time=np.array([s.time for s in end]),
                     rejected=np.array([s.rejected for s in end]))
     ctx, out = state["ctx"], state["out"]
