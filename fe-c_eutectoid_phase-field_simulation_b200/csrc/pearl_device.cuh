@@ -352,47 +352,47 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 constexpr unsigned long long kBarrierTimeoutNs = 4000000000ull;  // 4 s; a phase takes well under 0.1 s
 
 // Grid barrier for a cooperative launch (all blocks are co-resident) on one
-// monotonic 64-bit arrival counter: a block's arrival ticket names its
-// barrier, which completes when the counter reaches the next multiple of the
-// block count, so there is no reset and no second word on the critical path
-// (one atomic and one polled load per block; against a count-and-generation
-// pair this took 19 % off a 256x512 step and 1 % off a 2048x4096 one).  The
-// wait is bounded: after kBarrierTimeoutNs the block records
-// PEARL_ERR_DEVICE_WAIT and every caller returns without further device work;
-// the host zeroes the counter before the next launch.  Ordering: block
-// barrier, arrival with release (and acquire) semantics at GPU scope, polling
-// with acquire loads, block barrier.
-__device__ __forceinline__ unsigned long long atom_add_acq_rel_gpu(unsigned long long* p, unsigned long long v) {
-    unsigned long long old;
-    asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
-    return old;
+// monotonic 64-bit arrival counter: barrier number k (from 0) of a launch
+// completes when the counter reaches (k + 1) x blocks, so there is no reset
+// and, the number being known to the block, no ticket: an arrival is a
+// reduction without a result, and polling starts at once instead of after an
+// atomic's round trip.  The wait is bounded: after kBarrierTimeoutNs the block
+// records PEARL_ERR_DEVICE_WAIT and every caller returns without further
+// device work; the host zeroes the counter before the next launch.  Ordering:
+// block barrier, arrival with release semantics at GPU scope, polling with
+// acquire loads by the warp that then reads, block barrier.  (Arrivals spread
+// over eight counters that the lanes watch side by side measured 0.0569
+// against 0.0546 ms a step on 256x512; relaxed polls with one fence after the
+// last 0.0678.)
+__device__ __forceinline__ void arrive_release_gpu(unsigned long long* p) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(1ull) : "memory");
 }
 __device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned nblocks) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        // the k-th barrier of the launch completes when the counter reaches k * nblocks
-        const unsigned long long n = nblocks;
-        const unsigned long long target = (atom_add_acq_rel_gpu(&ctl->bar_count, 1ull) / n + 1) * n;
-        const unsigned long long t0 = globaltimer_ns();
-        unsigned spins = 0;
-        while (ld_acquire_gpu(&ctl->bar_count) < target) {
-            if ((++spins & 255u) == 0 && globaltimer_ns() - t0 > kBarrierTimeoutNs) {
-                ok = 0;
-                atomicCAS(&ctl->status, 0, (int)PEARL_ERR_DEVICE_WAIT);
-                break;
-            }
+// One lane's wait.
+__device__ __forceinline__ bool wait_arrivals(Ctl* ctl, unsigned long long target) {
+    unsigned spins = 0;
+    unsigned long long t0 = 0;  // set at the first check: a wait that ends soon reads no timer
+    while (ld_acquire_gpu(&ctl->bar_count) < target) {
+        if ((++spins & 255u) != 0) continue;
+        const unsigned long long t = globaltimer_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kBarrierTimeoutNs) {
+            atomicCAS(&ctl->status, 0, (int)PEARL_ERR_DEVICE_WAIT);
+            return false;
         }
-        s_ok = ok;
     }
-    __syncthreads();
-    return s_ok != 0;
+    return true;
+}
+// The block's first warp: arrive at barrier `number` of the launch and wait for
+// all blocks.  The vote makes the outcome the warp's, and brings the lanes
+// together again, whatever poll each left the loop at.
+__device__ __forceinline__ bool warp_grid_barrier(Ctl* ctl, int nblk, unsigned long long number) {
+    if ((threadIdx.x & 31) == 0) arrive_release_gpu(&ctl->bar_count);
+    return __all_sync(0xffffffffu, wait_arrivals(ctl, (number + 1) * (unsigned long long)nblk));
 }
 
 // ---------------------------------------------------------------- reductions
@@ -402,59 +402,93 @@ __device__ __forceinline__ bool grid_barrier(Ctl* ctl, unsigned nblocks) {
 enum RedOp : unsigned { kSum = 0, kMax = 1, kMin = 2 };
 
 __device__ __forceinline__ double red_apply(unsigned op, double a, double b) {
-    // fmax/fmin drop NaN like the reference's std::max(acc, v)/std::min(acc, v)
-    return op == kSum ? a + b : (op == kMax ? fmax(a, b) : fmin(a, b));
+    // max and min keep the accumulator unless b is beyond it, which drops a NaN b
+    // like the reference's std::max(acc, v)/std::min(acc, v); no accumulator is NaN
+    return op == kSum ? a + b : (op == kMax ? (b > a ? b : a) : (b < a ? b : a));
 }
 __device__ __forceinline__ double red_identity(unsigned op) {
     return op == kSum ? 0.0 : (op == kMax ? -INFINITY : INFINITY);
 }
 __device__ __forceinline__ unsigned op_of(unsigned ops, int k) { return (ops >> (2 * k)) & 3u; }
 
+// One value's block partials combined by a warp: lane l adds those of blocks
+// l, l + 32, ... in order, then a shuffle tree; lane 0 returns the result.  Ten
+// loads in flight cover a grid of 320 blocks in one round trip to L2.  An
+// absent partial contributes the identity, which changes no bit (a sum that
+// starts at +0 is never -0).
+__device__ __forceinline__ double gather_partials(unsigned op, const double* partials, int nblk) {
+    constexpr int kAhead = 10;
+    const int lane = threadIdx.x & 31;
+    double acc = red_identity(op);
+    for (int b = lane; b < nblk; b += 32 * kAhead) {
+        double t[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+            t[j] = b + 32 * j < nblk ? __ldcg(partials + b + 32 * j) : red_identity(op);
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) acc = red_apply(op, acc, t[j]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = red_apply(op, acc, __shfl_down_sync(0xffffffffu, acc, o));
+    return acc;
+}
+
 namespace PEARL_GEOM_NS {  // the block's warps
+// One grid reduction: barrier number `number` of the launch, block partials in
+// part_slot[value][block].  False after a bounded wait ran out.
+//
+// Latency is all that counts here (a step of a small domain is a chain of a
+// dozen of these), so the way from the last cell to the combined value is kept
+// short: the values' shuffle trees run side by side, one lane per value combines
+// the warps, the first warp alone arrives and polls, and then one warp per value
+// gathers that value's partials, which are contiguous.  With the arrival above
+// this took a step of 128x256 from 0.0758 to 0.0582 ms, of 256x512 from 0.0632
+// to 0.0546 and of 512x1024 from 0.188 to 0.151 (1965 MHz): before, one warp
+// gathered value after value, and FINAL's five cost it 4 us at 256 blocks.
 template <int NV>
-__device__ __forceinline__ void block_publish(const double (&v)[NV], unsigned ops, double* part_slot, int bid) {
-    __shared__ double s_red[kThreads / 32][kMaxRed];
+__device__ __forceinline__ bool grid_reduce(double (&v)[NV], unsigned ops, double* part_slot, int bid, int nblk,
+                                            Ctl* ctl, unsigned long long number) {
+    __shared__ double s_red[kMaxRed][kThreads / 32];
+    __shared__ double s_out[kMaxRed];
+    __shared__ int s_ok;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const unsigned op = op_of(ops, k);
-        double t = v[k];
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t = red_apply(op, t, __shfl_down_sync(0xffffffffu, t, o));
-        if (lane == 0) s_red[warp][k] = t;
-    }
+        for (int k = 0; k < NV; ++k) v[k] = red_apply(op_of(ops, k), v[k], __shfl_down_sync(0xffffffffu, v[k], o));
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) s_red[k][warp] = v[k];
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
+        if (lane < NV) {
+            const unsigned op = op_of(ops, lane);
+            double acc = s_red[lane][0];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const unsigned op = op_of(ops, k);
-            double acc = s_red[0][k];
-            for (int w = 1; w < kThreads / 32; ++w) acc = red_apply(op, acc, s_red[w][k]);
-            part_slot[bid * kMaxRed + k] = acc;
+            for (int w = 1; w < kThreads / 32; ++w) acc = red_apply(op, acc, s_red[lane][w]);
+            part_slot[lane * nblk + bid] = acc;
+        }
+        __syncwarp();
+        const bool ok = warp_grid_barrier(ctl, nblk, number);
+        if (lane == 0) s_ok = ok;
+        if (NV == 1) {
+            const double t = gather_partials(ops & 3u, part_slot, nblk);
+            if (lane == 0) s_out[0] = t;
         }
     }
+    if (NV > 1) {
+        __syncthreads();
+        if (warp < NV) {
+            const double t = gather_partials(op_of(ops, warp), part_slot + warp * nblk, nblk);
+            if (lane == 0) s_out[warp] = t;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = s_out[k];
+    return s_ok != 0;
 }
 }  // namespace PEARL_GEOM_NS
-
-template <int NV>
-__device__ __forceinline__ void grid_gather(double (&out)[NV], unsigned ops, const double* part_slot, int nblk) {
-    __shared__ double s_out[kMaxRed];
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const unsigned op = op_of(ops, k);
-            double acc = red_identity(op);
-            for (int b = lane; b < nblk; b += 32) acc = red_apply(op, acc, part_slot[b * kMaxRed + k]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc = red_apply(op, acc, __shfl_down_sync(0xffffffffu, acc, o));
-            if (lane == 0) s_out[k] = acc;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) out[k] = s_out[k];
-    __syncthreads();
-}
 
 }  // namespace pearl_gpu

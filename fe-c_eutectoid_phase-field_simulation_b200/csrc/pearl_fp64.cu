@@ -255,11 +255,11 @@ struct PhaseClock {
 
 struct Red {
     const Dom& a;
-    PhaseClock* clk;  // shared memory; used by thread 0 of block 0 only
-    unsigned counter = 0;
+    PhaseClock* clk;  // shared memory; used by one thread of block 0 only (keeps_clock)
+    unsigned long long counter;  // grid reductions of this block group since the launch began
     struct Pipe* pipe_ptr = nullptr;
-    __device__ Red(const Dom& args, PhaseClock* c) : a(args), clk(c) {
-        if (a.bid == 0 && threadIdx.x == 0) {
+    __device__ Red(const Dom& args, PhaseClock* c, unsigned long long done = 0) : a(args), clk(c), counter(done) {
+        if (keeps_clock()) {
             clk->t_last = globaltimer_ns();
             for (int k = 0; k < kTagCount; ++k) {
                 clk->ns[k] = 0;
@@ -267,26 +267,27 @@ struct Red {
             }
         }
     }
+    // the second warp's first thread: the first warp is on the reduction's critical path
+    __device__ bool keeps_clock() const { return a.bid == 0 && threadIdx.x == 32; }
     // publish the block partials, wait for the grid, combine; false on a device-wait timeout
     template <int NV>
     __device__ bool reduce(double (&v)[NV], unsigned ops, int tag) {
         // this thread's plane stores may be read by TMA (async proxy) after the barrier
         if (a.use_tma) fence_proxy_async();
         double* slot = a.part + (size_t)(counter & 1u) * a.nblk * kMaxRed;
+        const bool ok = grid_reduce<NV>(v, ops, slot, a.bid, a.nblk, a.bar, counter);
         ++counter;
-        block_publish<NV>(v, ops, slot, a.bid);
-        if (!grid_barrier(a.bar, a.nblk)) return false;
-        if (a.bid == 0 && threadIdx.x == 0) {
+        if (!ok) return false;
+        if (keeps_clock()) {
             const unsigned long long t = globaltimer_ns();
             clk->ns[tag] += t - clk->t_last;
             clk->cnt[tag] += 1;
             clk->t_last = t;
         }
-        grid_gather<NV>(v, ops, slot, a.nblk);
         return true;
     }
     __device__ void flush() const {
-        if (a.bid == 0 && threadIdx.x == 0)
+        if (keeps_clock())
             for (int k = 0; k < kTagCount; ++k) {
                 a.B.ctl->phase_ns[k] = clk->ns[k];
                 a.B.ctl->phase_count[k] = clk->cnt[k];
@@ -479,19 +480,25 @@ __device__ bool sweep(const Dom& a, Pipe& pp, const int (&maps)[NF], const T* co
     };
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // plain stores of the earlier passes (ordered by the grid barrier) before the
-    // async reads of this sweep, by every thread that may issue copies (lane 0 of
-    // each warp), once per sweep: no value that a sweep stages and uses is changed
-    // by a plain store of the same sweep (a field written in a pass is either not
-    // staged in it, or read only at the cells that the reading block itself
-    // writes, after reading them)
-    if (lane == 0) fence_proxy_async();
-    // S-1 tiles ahead: the stage of tile k+S-1 is the one freed by the barrier ending tile k-1
-    if (threadIdx.x == 0)
+    // async reads of this sweep, by the thread that issues the copies, once per
+    // sweep: no value that a sweep stages and uses is changed by a plain store of
+    // the same sweep (a field written in a pass is either not staged in it, or
+    // read only at the cells that the reading block itself writes, after reading
+    // them).  S-1 tiles ahead: the stage of tile k+S-1 is the one freed by the
+    // barrier ending tile k-1.
+    if (threadIdx.x == 0) {
+        fence_proxy_async();
         for (int k = 0; k < S - 1 && k < nb; ++k) issue(k);
+    }
+    __syncwarp();
     for (int k = 0; k < nb; ++k) {
         const int s = k % S;
         if (threadIdx.x == 0 && k + S - 1 < nb) issue(k + S - 1);
-        if (!mbar_wait_bounded(&pp.bar[s], (pp.parity >> s) & 1u, kBarrierTimeoutNs, &a.bar->status)) {
+        // The lanes of a warp may see the stage arrive at different tries; the vote
+        // makes the outcome the warp's, and brings the lanes together before the
+        // block barriers below, which count warps.
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&pp.bar[s], (pp.parity >> s) & 1u, kBarrierTimeoutNs,
+                                                       &a.bar->status))) {
             atomicCAS(&a.bar->status, 0, (int)PEARL_ERR_DEVICE_WAIT);
             // drain the copies that may still be in flight, this tile's included
             // when the wait was cut short by another block's timeout, bounded
@@ -2105,6 +2112,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
     Ctl* gctl = args.group_ctl + g;
     double* gpart = args.group_part + (size_t)b0 * 2 * kMaxRed;
     const bool leader = bid == 0 && threadIdx.x == 0;
+    unsigned long long reductions = 0;  // of this group, over all its instances
     for (int j = args.first[g]; j < args.first[g + 1]; ++j) {
         const BatchInstance* I = args.inst + args.order[j];
         __syncthreads();
@@ -2114,7 +2122,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
         }
         __syncthreads();
         const Dom a{sP, sB, I->maps, args.use_tma, bid, nblk, gctl, gpart, 0, 0, 0, 0, 0, 0, 0};
-        Red red(a, &clk);
+        Red red(a, &clk, reductions);
         red.pipe_ptr = &pipe;
         Ctl* ctl = sB.ctl;
         StepState st;
@@ -2171,6 +2179,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
             gctl->why = 0;
         }
         red.flush();
+        reductions = red.counter;
     }
 }
 
@@ -2200,7 +2209,10 @@ __global__ void division_selftest_kernel(const double* a, const double* b, const
 // Self-test of the bounded grid-barrier wait: every block waits for one
 // arrival more than the grid has, so no wait can complete; each gives up after
 // kBarrierTimeoutNs and records PEARL_ERR_DEVICE_WAIT.
-__global__ void wait_limit_selftest_kernel(Ctl* ctl) { grid_barrier(ctl, gridDim.x + 1u); }
+__global__ void wait_limit_selftest_kernel(Ctl* ctl) {
+    __syncthreads();
+    if (threadIdx.x < 32) warp_grid_barrier(ctl, (int)gridDim.x + 1, 0);
+}
 
 #include "pearl_adjoint.cuh"
 
