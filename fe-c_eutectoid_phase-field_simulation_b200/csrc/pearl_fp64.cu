@@ -253,8 +253,53 @@ struct PhaseClock {
     unsigned cnt[kTagCount];
 };
 
+// ------------------------------------------------------------------ uniform tiles
+// Most of a domain is austenite ahead of the front, where neighbouring cells
+// are equal bit for bit: every pass then computes one and the same value at
+// every cell of a tile.  PROPOSE, which reads the whole state anyway, finds the
+// tiles whose cells and one-cell surroundings all equal one reference cell in
+// phi, mu and carbon (by bit pattern).  In the passes of the implicit solve
+// that value is computed once per block (Uniform), the tile's threads add it to
+// their running sums in the tile's place of the walk, and the tile's work planes
+// are neither read nor written: 104 bytes a cell and step instead of about 950.
+// Sums keep their order and cells their arithmetic, so every result is the same
+// bit for bit; a domain without uniform tiles takes the dense path throughout.
+//
+// What is not uniform spreads one cell per conjugate-gradient iteration, so a
+// tile beside a non-uniform one is dense as well (the rim), and a tile beside
+// the rim writes the planes that the rim reads at its edge (the border).  The
+// rim is as thick as a tile's shorter side (kReach cells): a solve that takes
+// more iterations than that writes the uniform tiles' planes and goes on dense
+// (phase_expand).  Tiles at the two walls are dense, their diagonal differs.
+enum TileClass : unsigned char { kDense = 0, kUniform = 1, kBorder = 2, kClassMask = 3, kLastColumn = 4 };
+// Fewer tile rows leave nothing between the walls' rims and the front's.
+constexpr int kMinTileRowsUniform = 8;
+constexpr int kMaxListedTiles = 2048;  // tiles of one block; a block with more runs dense
+constexpr int kReach = kTileRows < kTileX ? kTileRows : kTileX;
+
+// The value of every cell of a uniform tile, and what the passes make of it.
+struct Uniform {
+    double ref[5];            // the reference cell: phi (3), mu, carbon
+    double q0, q1, q2, change;  // its proposal
+    double K, chi, icpt;
+    int have, simplex_bad, mix_bad;
+    Faces f;
+    double x, r, z, p, Ap, diag, cn, mun, closure;
+    double add[3];  // the cell's contributions to the current pass's sums
+    int bad;
+};
+struct Tiles {
+    int enabled;  // this launch looks for uniform tiles
+    int active;   // cls and list describe the current attempt
+    int ndense;
+    Uniform u;
+    unsigned char cls[kMaxListedTiles];    // TileClass of the block's tiles, in walk order
+    unsigned short list[kMaxListedTiles];  // positions of the dense ones
+};
+
 struct Red {
     const Dom& a;
+    Tiles* tiles = nullptr;  // shared memory
     PhaseClock* clk;  // shared memory; used by one thread of block 0 only (keeps_clock)
     unsigned long long counter;  // grid reductions of this block group since the launch began
     struct Pipe* pipe_ptr = nullptr;
@@ -438,9 +483,34 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // passes that alternate direction begin where the previous pass ended, on
 // tiles whose planes are still in L2.  The direction is fixed per phase, so
 // a run's sums do not depend on how it is split into launches.
-template <int NF, bool kTileOnly = false, class T = double, class Body>
-__device__ bool sweep(const Dom& a, Pipe& pp, const int (&maps)[NF], const T* const (&planes)[NF],
-                      unsigned stencil, bool reverse, Body&& body) {
+// `uni` is the pass's part for uniform tiles (NoUniform: it has none): when the
+// attempt's tiles are classified, uni.prepare() runs in one thread while the
+// first copies are under way, and uni.tile(k, valid) takes the place of the
+// dense tile; `tile_end(t)` replaces the block barrier that ends a tile.
+struct NoUniform {
+    static constexpr bool kAny = false;
+    __device__ void prepare() const {}
+    __device__ void tile(int, int, bool) const {}
+};
+template <bool kHas, class Prepare, class Tile>
+struct UniformPass {
+    static constexpr bool kAny = kHas;
+    Prepare prepare_;
+    Tile tile_;
+    __device__ void prepare() const { prepare_(); }
+    __device__ void tile(int t, int cls, bool valid) const { tile_(t, cls, valid); }
+};
+template <bool kHas, class Prepare, class Tile>
+__device__ __forceinline__ UniformPass<kHas, Prepare, Tile> uniform_pass(Prepare p, Tile t) {
+    return {p, t};
+}
+struct BlockBarrier {
+    __device__ void operator()(int) const { __syncthreads(); }
+};
+template <int NF, bool kTileOnly = false, class T = double, class Body, class Uni = NoUniform, class End = BlockBarrier>
+__device__ bool sweep(const Dom& a, Red& red, const int (&maps)[NF], const T* const (&planes)[NF],
+                      unsigned stencil, bool reverse, Body&& body, Uni&& uni = Uni{}, End&& tile_end = End{}) {
+    Pipe& pp = *red.pipe_ptr;
     using G_ = StageGeom<T>;
     const DevParams& P = a.P;
     const int G = a.nblk;
@@ -464,10 +534,23 @@ __device__ bool sweep(const Dom& a, Pipe& pp, const int (&maps)[NF], const T* co
                           : kMaxStages;
     static_assert(S >= 2, "pipeline needs two stages");
     T* const stage = reinterpret_cast<T*>(pp.stage);
-    const auto issue = [&](int k) {  // one thread
-        const int t = tile_of(k);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // plain stores of the earlier passes (ordered by the grid barrier) before the
+    // async reads of this sweep, by the thread that issues the copies, once per
+    // sweep: no value that a sweep stages and uses is changed by a plain store of
+    // the same sweep (a field written in a pass is either not staged in it, or
+    // read only at the cells that the reading block itself writes, after reading
+    // them).  S-1 tiles ahead: the stage of tile k+S-1 is the one freed by the
+    // barrier ending tile k-1.
+    const bool skip = std::remove_reference_t<Uni>::kAny && red.tiles->active;
+    const int nd = skip ? red.tiles->ndense : nb;  // dense tiles, staged in walk order
+    const auto dense_at = [&](int d) {
+        return !skip ? d : reverse ? nb - 1 - (int)red.tiles->list[nd - 1 - d] : (int)red.tiles->list[d];
+    };
+    const auto issue = [&](int d) {  // one thread
+        const int t = tile_of(dense_at(d));
         const int bx = t % P.ntx, by = t / P.ntx;
-        const int s = k % S;
+        const int s = d % S;
         T* dst = stage + (size_t)s * NF * G_::kStride;
         // tile-only boxes start at the tile (x multiple of 32 cells); halo boxes
         // kHaloX cells left, one row up
@@ -478,22 +561,32 @@ __device__ bool sweep(const Dom& a, Pipe& pp, const int (&maps)[NF], const T* co
             tma_load_2d(dst + f * G_::kStride, &a.maps[maps[f]], bx * kTileX - (kTileOnly ? 0 : G_::kHaloX),
                         by * kTileRows - (kTileOnly ? 0 : 1), &pp.bar[s]);
     };
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // plain stores of the earlier passes (ordered by the grid barrier) before the
-    // async reads of this sweep, by the thread that issues the copies, once per
-    // sweep: no value that a sweep stages and uses is changed by a plain store of
-    // the same sweep (a field written in a pass is either not staged in it, or
-    // read only at the cells that the reading block itself writes, after reading
-    // them).  S-1 tiles ahead: the stage of tile k+S-1 is the one freed by the
-    // barrier ending tile k-1.
     if (threadIdx.x == 0) {
         fence_proxy_async();
-        for (int k = 0; k < S - 1 && k < nb; ++k) issue(k);
+        for (int d = 0; d < S - 1 && d < nd; ++d) issue(d);
     }
     __syncwarp();
-    for (int k = 0; k < nb; ++k) {
-        const int s = k % S;
-        if (threadIdx.x == 0 && k + S - 1 < nb) issue(k + S - 1);
+    if constexpr (std::remove_reference_t<Uni>::kAny) {
+        if (skip) {
+            if (threadIdx.x == 32) uni.prepare();
+            __syncthreads();
+        }
+    }
+    int done = 0;  // tiles of the walk so far
+    for (int d = 0; d < nd || skip; ++d) {
+        const int k = d < nd ? dense_at(d) : nb;
+        if (threadIdx.x == 0 && d + S - 1 < nd) issue(d + S - 1);
+        if constexpr (std::remove_reference_t<Uni>::kAny) {
+            if (skip) {
+                for (; done < k; ++done) {
+                    const unsigned char c = red.tiles->cls[reverse ? nb - 1 - done : done];
+                    uni.tile(tile_of(done), c & kClassMask, !(c & kLastColumn) || lane < P.nx - (P.ntx - 1) * kTileX);
+                }
+                if (d >= nd) break;
+                ++done;
+            }
+        }
+        const int s = d % S;
         // The lanes of a warp may see the stage arrive at different tries; the vote
         // makes the outcome the warp's, and brings the lanes together before the
         // block barriers below, which count warps.
@@ -502,7 +595,7 @@ __device__ bool sweep(const Dom& a, Pipe& pp, const int (&maps)[NF], const T* co
             atomicCAS(&a.bar->status, 0, (int)PEARL_ERR_DEVICE_WAIT);
             // drain the copies that may still be in flight, this tile's included
             // when the wait was cut short by another block's timeout, bounded
-            for (int j = k; j < nb && j < k + S; ++j)
+            for (int j = d; j < nd && j < d + S; ++j)
                 mbar_wait_bounded(&pp.bar[j % S], (pp.parity >> (j % S)) & 1u, kBarrierTimeoutNs / 16);
             return false;
         }
@@ -531,7 +624,7 @@ __device__ bool sweep(const Dom& a, Pipe& pp, const int (&maps)[NF], const T* co
                           : SmemSrc<NF, T>{st, lane + G_::kHaloX, 2 * warp + 1, c.y0 > 0, c.v1, c.y0 + 2 < P.ny, G_::kW};
             body(src, c);
         }
-        __syncthreads();  // every warp is done with stage s: it is refilled next iteration
+        tile_end(t);  // every warp is done with stage s: it is refilled next iteration
     }
     return true;
 }
@@ -665,18 +758,75 @@ __device__ __forceinline__ Proposal propose_cell_mixed(const DevParams& P, const
 // the trial phi (K, chi, icpt); in phase_only mode also the reconstructed
 // trial carbon and the copied trial mu (pearl_serial.cpp:1134-1136).
 // Reduction: {max |dphi| (inf if non-finite), mixture invalid, simplex failed}.
+// With kFindUniform it also finds the uniform tiles (Tiles): carbon is staged
+// beside phi and mu for that, 8 bytes a cell in a phase that its arithmetic
+// bounds.  A cell that equals the reference cell with its neighbours takes the
+// proposal computed at the first such cell of the block.
+template <bool kFindUniform>
 __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double& change, bool& mixbad,
                               bool& simplexbad) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     double* const* tp = B.phi[cur ^ 1];
     double vchange = 0, vmix = 0, vsimp = 0;
-    const int maps[4] = {kMapState + 5 * cur, kMapState + 5 * cur + 1, kMapState + 5 * cur + 2,
-                         kMapState + 5 * cur + 4};
-    const double* const planes[4] = {B.phi[cur][0], B.phi[cur][1], B.phi[cur][2], B.mu[cur]};
+    constexpr int NF = kFindUniform ? 5 : 4;
+    constexpr unsigned kWrapped = kFindUniform ? 0xFu : 0x7u;  // fields read across the periodic edge
+    int maps[NF] = {kMapState + 5 * cur, kMapState + 5 * cur + 1, kMapState + 5 * cur + 2, kMapState + 5 * cur + 4};
+    const double* planes[NF] = {B.phi[cur][0], B.phi[cur][1], B.phi[cur][2], B.mu[cur]};
+    const bool find = kFindUniform && red.tiles->enabled;
+    Uniform& U = red.tiles->u;
+    bool same = true, have = false;  // this thread's cells of the tile are uniform; U holds their proposal
+    if constexpr (kFindUniform) {
+        maps[4] = kMapState + 5 * cur + 3;
+        planes[4] = B.c[cur];
+        if (find) {
+            // reference cell: some rows below the top wall, where the austenite has been longest
+            const size_t i = (size_t)(P.ny - 1 - P.ny / 16) * P.pitch + P.nx / 2;
+            if (threadIdx.x < 5) U.ref[threadIdx.x] = planes[threadIdx.x][i];
+            if (threadIdx.x == 0) {
+                U.have = 0;
+                red.tiles->active = 0;
+            }
+            __syncthreads();
+        }
+    }
+    const auto equals_ref = [&](const auto& src, const Pair& c) {
+        if (c.y0 < kTileRows || c.y0 / kTileRows == P.nty - 1) return false;  // the tiles at the walls
+        const auto differs = [&](double v, double ref) { return __double_as_longlong(v) ^ __double_as_longlong(ref); };
+        long long d = differs(src.v(2, 0, kC), U.ref[2]);
+        if (d) return false;
+        if constexpr (kFindUniform) d = differs(src.v(4, 0, kC), U.ref[4]) | differs(src.v(4, 1, kC), U.ref[4]);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            const double r = U.ref[f];
+            d |= differs(src.v(f, 0, kC), r) | differs(src.v(f, 1, kC), r) | differs(src.v(f, 0, kW), r) |
+                 differs(src.v(f, 0, kE), r) | differs(src.v(f, 1, kW), r) | differs(src.v(f, 1, kE), r) |
+                 differs(src.v(f, 0, kS), r) | differs(src.v(f, 1, kN), r);
+        }
+        return d == 0;
+    };
     // the FP64 and the mixed-precision proposal are separate sweeps, so each
     // loop is register-allocated on its own
     const auto body = [&](auto mixed_tag, const auto& src, const Pair& c) {
+        if (find) {
+            same = equals_ref(src, c);
+            if (same && have) {
+                vchange = fmax(vchange, U.change);
+                if (U.simplex_bad) vsimp = 1;
+                if (U.mix_bad) vmix = 1;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const size_t i = k ? c.i1 : c.i0;
+                    tp[0][i] = U.q0;
+                    tp[1][i] = U.q1;
+                    tp[2][i] = U.q2;
+                    B.K[i] = U.K;
+                    B.chi[i] = U.chi;
+                    B.icpt[i] = U.icpt;
+                }
+                return;
+            }
+        }
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {
             if (k == 1 && !c.v1) break;
@@ -693,22 +843,46 @@ __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double
             tp[1][i] = o.z1;
             tp[2][i] = o.z2;
             double chi, cint, K;
-            if (!mixture(P, o.z0, o.z1, o.z2, chi, cint, K)) vmix = 1;
+            const bool mix = mixture(P, o.z0, o.z1, o.z2, chi, cint, K);
+            if (!mix) vmix = 1;
+            const double icpt = fma(chi, P.mu_ref, cint);
             B.K[i] = K;
             B.chi[i] = chi;
-            B.icpt[i] = fma(chi, P.mu_ref, cint);
+            B.icpt[i] = icpt;
             if (P.phase_only) {
                 const double mu = src.v(3, k, kC);
                 B.c[cur ^ 1][i] = fma(chi, mu, cint);
                 B.mu[cur ^ 1][i] = mu;
             }
+            if (kFindUniform && find && same && k == 0 && threadIdx.x == 0) {
+                U.q0 = o.z0;
+                U.q1 = o.z1;
+                U.q2 = o.z2;
+                U.change = o.change;
+                U.simplex_bad = o.simplex_bad;
+                U.mix_bad = !mix;
+                U.K = K;
+                U.chi = chi;
+                U.icpt = icpt;
+                U.have = 1;
+            }
         }
     };
+    const auto tile_end = [&](int t) {
+        if (!find) {
+            __syncthreads();
+            return;
+        }
+        const int all = __syncthreads_and(same);
+        if (threadIdx.x == 0) B.mixed_tile[t] = !all;
+        same = true;  // lanes outside the domain have no say
+        if (!have) have = U.have != 0;
+    };
     const bool ok =
-        P.mixed ? sweep<4>(a, *red.pipe_ptr, maps, planes, 0x7u, true,
-                           [&](const auto& src, const Pair& c) { body(std::true_type{}, src, c); })
-                : sweep<4>(a, *red.pipe_ptr, maps, planes, 0x7u, true,
-                           [&](const auto& src, const Pair& c) { body(std::false_type{}, src, c); });
+        P.mixed ? sweep<NF>(a, red, maps, planes, kWrapped, true,
+                            [&](const auto& src, const Pair& c) { body(std::true_type{}, src, c); }, NoUniform{}, tile_end)
+                : sweep<NF>(a, red, maps, planes, kWrapped, true,
+                            [&](const auto& src, const Pair& c) { body(std::false_type{}, src, c); }, NoUniform{}, tile_end);
     if (!ok) return false;
     double v[3] = {vchange, vmix, vsimp};
     if (!red.reduce<3>(v, OPS3(kMax, kMax, kMax), kTagPropose)) return false;
@@ -716,6 +890,52 @@ __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double
     mixbad = v[1] != 0;
     simplexbad = v[2] != 0;
     return true;
+}
+
+// The classes of the block's tiles for the current attempt, from the marks that
+// PROPOSE left (all blocks', after its reduction).  A tile within one tile of a
+// marked one is dense, within two a border tile; a last column narrower than
+// the rim counts with the column beyond it (x is periodic).
+__device__ void classify_tiles(const Dom& a, Tiles& T) {
+    const DevParams& P = a.P;
+    const int nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
+    const int rest = P.nx - (P.ntx - 1) * kTileX, thin = rest < kReach ? 1 : 0;
+    for (int k = threadIdx.x; k < nb; k += kThreads) {
+        const int t = a.bid + k * a.nblk, bx = t % P.ntx, by = t / P.ntx;
+        const unsigned char* m = a.B.mixed_tile;
+        int nearest = 3;
+        // all marks at once: none of the loads waits for another's outcome
+#pragma unroll
+        for (int dy = -2; dy <= 2; ++dy) {
+            const int y = min(max(by + dy, 0), P.nty - 1);  // beyond a wall: the wall's own row, marked and nearer
+#pragma unroll
+            for (int dx = -3; dx <= 3; ++dx) {
+                int x = bx + dx;
+                while (x < 0) x += P.ntx;
+                while (x >= P.ntx) x -= P.ntx;
+                const int far = max(abs(dy), max(abs(dx) - thin, 0));
+                if (m[(size_t)y * P.ntx + x]) nearest = min(nearest, far);
+            }
+        }
+        T.cls[k] = (unsigned char)((nearest <= 1 ? kDense : nearest == 2 ? kBorder : kUniform) |
+                                   (bx == P.ntx - 1 ? kLastColumn : 0));
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int n = 0;
+        for (int k0 = 0; k0 < nb; k0 += 32) {
+            const int k = k0 + threadIdx.x;
+            const bool dense = k < nb && (T.cls[k] & kClassMask) == kDense;
+            const unsigned votes = __ballot_sync(0xffffffffu, dense);
+            if (dense) T.list[n + __popc(votes & ((1u << threadIdx.x) - 1))] = (unsigned short)k;
+            n += __popc(votes);
+        }
+        if (threadIdx.x == 0) {
+            T.ndense = n;
+            T.active = 1;
+        }
+    }
+    __syncthreads();
 }
 
 // MIX: K, chi, icpt of the trial phi (used when the trial phi was uploaded).
@@ -753,7 +973,41 @@ __device__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& 
     double s0 = 0, s1 = 0, s2 = 0;
     const int maps[5] = {kMapK, kMapState + 5 * cur + 4, kMapChi, kMapIcpt, kMapState + 5 * cur + 3};
     const double* const planes[5] = {B.K, B.mu[cur], B.chi, B.icpt, B.c[cur]};
-    const bool ok = sweep<5>(a, *red.pipe_ptr, maps, planes, 0x3u, false, [&](const auto& src, const Pair& c) {
+    Uniform& U = red.tiles->u;
+    const auto uni = uniform_pass<!kSolve32>(
+        [&] {
+            U.x = U.ref[3] - P.mu_ref;
+            const double wx = face_x(P, U.K, U.K), wy = face_y(P, U.K, U.K);
+            U.f = Faces{wx, wx, wy, wy};
+            const double Au = apply_at(U.chi, dt, U.f, U.x, U.x, U.x, U.x, U.x);
+            U.diag = U.chi + dt * (U.f.w0 + U.f.w1 + U.f.w2 + U.f.w3);
+            const double rhs = U.ref[4] - U.icpt;
+            U.r = rhs - Au;
+            U.z = U.r / U.diag;
+            U.add[0] = rhs * rhs;
+            U.add[1] = U.r * U.z;
+            U.add[2] = U.r * U.r;
+        },
+        [&](int t, int cls, bool valid) {
+            if (!valid) return;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                s0 += U.add[0];
+                s1 += U.add[1];
+                s2 += U.add[2];
+            }
+            if (cls != kBorder) return;
+            const Pair c = pair_of(P, t);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const size_t i = k ? c.i1 : c.i0;
+                B.wE[i] = U.f.w1;
+                B.wN[i] = U.f.w3;
+                B.x[i] = U.x;
+                B.z[i] = U.z;
+            }
+        });
+    const bool ok = sweep<5>(a, red, maps, planes, 0x3u, false, [&](const auto& src, const Pair& c) {
         const S2 K = stencil2(src, 0, c.v1);
         S2 u = stencil2(src, 1, c.v1);
         u.c0 -= P.mu_ref; u.c1 -= P.mu_ref; u.w0 -= P.mu_ref; u.e0 -= P.mu_ref;
@@ -800,7 +1054,7 @@ __device__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& 
             const double rhs = cold - ic;
             store(c.i1, chi, f, u.c1, rhs, rhs - Au, diag);
         }
-    });
+    }, uni);
     if (!ok) return false;
     double v[3] = {s0, s1, s2};
     if (!red.reduce<3>(v, OPS3(kSum, kSum, kSum), kTagSetup)) return false;
@@ -840,15 +1094,31 @@ __device__ bool phase_apply(const Dom& a, Red& red, double dt, bool first, doubl
             s += p.c1 * Ap1;
         }
     };
+    Uniform& U = red.tiles->u;
+    const auto uni = uniform_pass<true>(
+        [&] {
+            U.p = first ? U.z : U.z + beta * U.p;
+            U.Ap = apply_at(U.chi, dt, U.f, U.p, U.p, U.p, U.p, U.p);
+            U.add[0] = U.p * U.Ap;
+        },
+        [&](int t, int cls, bool valid) {
+            if (!valid) return;
+            s += U.add[0];
+            s += U.add[0];
+            if (cls != kBorder) return;
+            const Pair c = pair_of(a.P, t);
+            pn[c.i0] = U.p;
+            pn[c.i1] = U.p;
+        });
     bool ok;
     if (first) {
         const int maps[4] = {kMapWE, kMapWN, kMapZ, kMapChi};
         const double* const planes[4] = {B.wE, B.wN, B.z, B.chi};
-        ok = sweep<4>(a, *red.pipe_ptr, maps, planes, 0x7u, true, body);
+        ok = sweep<4>(a, red, maps, planes, 0x7u, true, body, uni);
     } else {
         const int maps[5] = {kMapWE, kMapWN, kMapZ, kMapChi, pout ? kMapP0 : kMapP1};
         const double* const planes[5] = {B.wE, B.wN, B.z, B.chi, B.p[pout ^ 1]};
-        ok = sweep<5>(a, *red.pipe_ptr, maps, planes, 0x17u, true, body);
+        ok = sweep<5>(a, red, maps, planes, 0x17u, true, body, uni);
     }
     if (!ok) return false;
     double v[1] = {s};
@@ -864,7 +1134,28 @@ __device__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, dou
     double s0 = 0, s1 = 0;
     const int maps[5] = {kMapXc, pcur ? kMapP1c : kMapP0c, kMapRc, kMapApc, kMapDiagc};
     const double* const planes[5] = {B.x, B.p[pcur], B.r, B.Ap, B.diag};
-    const bool ok = sweep<5, true>(a, *red.pipe_ptr, maps, planes, 0x0u, false, [&](const auto& src, const Pair& c) {
+    Uniform& U = red.tiles->u;
+    const auto uni = uniform_pass<true>(
+        [&] {
+            U.x = U.x + alpha * U.p;
+            U.r = U.r - alpha * U.Ap;
+            U.z = U.r / U.diag;
+            U.add[0] = U.r * U.z;
+            U.add[1] = U.r * U.r;
+        },
+        [&](int t, int cls, bool valid) {
+            if (!valid) return;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                s0 += U.add[0];
+                s1 += U.add[1];
+            }
+            if (cls != kBorder) return;
+            const Pair c = pair_of(a.P, t);
+            B.x[c.i0] = B.x[c.i1] = U.x;
+            B.z[c.i0] = B.z[c.i1] = U.z;
+        });
+    const bool ok = sweep<5, true>(a, red, maps, planes, 0x0u, false, [&](const auto& src, const Pair& c) {
         {
             const double x = src.v(0, 0, kC) + alpha * src.v(1, 0, kC), r = src.v(2, 0, kC) - alpha * src.v(3, 0, kC);
             const double z = r / src.v(4, 0, kC);
@@ -883,7 +1174,7 @@ __device__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, dou
             s0 += r * z;
             s1 += r * r;
         }
-    });
+    }, uni);
     if (!ok) return false;
     double v[2] = {s0, s1};
     if (!red.reduce<2>(v, OPS2(kSum, kSum), kTagUpdate)) return false;
@@ -897,20 +1188,58 @@ __device__ bool phase_reset(const Dom& a, Red& red, double& rz) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     double s = 0;
+    const Tiles& T = *red.tiles;
+    const bool skip = T.active;
+    if (skip) {
+        if (threadIdx.x == 0) red.tiles->u.z = T.u.r / T.u.diag;
+        __syncthreads();
+    }
+    int pos = 0;
     FOR_TILES(P) {
         const Pair c = pair_of(P, t);
+        const int cls = skip ? T.cls[pos] & kClassMask : kDense;
+        ++pos;
         for (int k = 0; k < 2; ++k) {
             if (!(k ? c.v1 : c.v0)) continue;
             const size_t i = k ? c.i1 : c.i0;
-            const double r = B.r[i];
-            const double z = r / B.diag[i];
-            B.z[i] = z;
+            const double r = cls == kDense ? B.r[i] : T.u.r;
+            const double z = cls == kDense ? r / B.diag[i] : T.u.z;
+            if (cls != kUniform) B.z[i] = z;
             s += r * z;
         }
     }
     double v[1] = {s};
     if (!red.reduce<1>(v, kSum, kTagReset)) return false;
     rz = v[0];
+    return true;
+}
+
+// EXPAND: a solve whose search direction has spread through the rim writes the
+// planes of its uniform and border tiles and goes on dense (see Tiles).
+__device__ bool phase_expand(const Dom& a, Red& red, int pcur) {
+    const DevParams& P = a.P;
+    const DevBufs& B = a.B;
+    const Uniform& U = red.tiles->u;
+    int pos = 0;
+    FOR_TILES(P) {
+        if ((red.tiles->cls[pos++] & kClassMask) == kDense) continue;
+        const Pair c = pair_of(P, t);
+        for (int k = 0; k < 2; ++k) {
+            if (!(k ? c.v1 : c.v0)) continue;
+            const size_t i = k ? c.i1 : c.i0;
+            B.wE[i] = U.f.w1;
+            B.wN[i] = U.f.w3;
+            B.diag[i] = U.diag;
+            B.x[i] = U.x;
+            B.r[i] = U.r;
+            B.z[i] = U.z;
+            B.p[pcur][i] = U.p;
+        }
+    }
+    double v[1] = {0};
+    if (!red.reduce<1>(v, kMax, kTagReset)) return false;
+    if (threadIdx.x == 0) red.tiles->active = 0;
+    __syncthreads();
     return true;
 }
 
@@ -1007,11 +1336,11 @@ __device__ bool phase_apply32(const Dom& a, Red& red, double dt, bool first, dou
     if (first) {
         const int maps[4] = {kMap32WE, kMap32WN, kMap32Z, kMap32Chi};
         const float* const planes[4] = {B.wE32, B.wN32, B.z32, B.chi32};
-        ok = sweep<4, false, float>(a, *red.pipe_ptr, maps, planes, 0x7u, true, body);
+        ok = sweep<4, false, float>(a, red, maps, planes, 0x7u, true, body);
     } else {
         const int maps[5] = {kMap32WE, kMap32WN, kMap32Z, kMap32Chi, pout ? kMap32P0 : kMap32P1};
         const float* const planes[5] = {B.wE32, B.wN32, B.z32, B.chi32, B.p32[pout ^ 1]};
-        ok = sweep<5, false, float>(a, *red.pipe_ptr, maps, planes, 0x17u, true, body);
+        ok = sweep<5, false, float>(a, red, maps, planes, 0x17u, true, body);
     }
     if (!ok) return false;
     double v[1] = {s};
@@ -1085,7 +1414,7 @@ __device__ bool phase_resid32(const Dom& a, Red& red, int cur, double dt, double
     double s0 = 0, s1 = 0;
     const int maps[6] = {kMapWE, kMapWN, kMapX, kMapChi, kMapState + 5 * cur + 3, kMapIcpt};
     const double* const planes[6] = {B.wE, B.wN, B.x, B.chi, B.c[cur], B.icpt};
-    const bool ok = sweep<6>(a, *red.pipe_ptr, maps, planes, 0x7u, true, [&](const auto& src, const Pair& c) {
+    const bool ok = sweep<6>(a, red, maps, planes, 0x7u, true, [&](const auto& src, const Pair& c) {
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {
             if (k == 1 && !c.v1) break;
@@ -1151,7 +1480,36 @@ __device__ bool phase_final(const Dom& a, Red& red, int cur, double dt, double& 
                          kMapState + 5 * cur + 3, kMapChi, kMapIcpt};
     const double* const planes[9] = {B.wE, B.wN, B.x, B.phi[tr][0], B.phi[tr][1], B.phi[tr][2], B.c[cur], B.chi,
                                      B.icpt};
-    const bool ok = sweep<9>(a, *red.pipe_ptr, maps, planes, 0x3Fu, true, [&](const auto& src, const Pair& c) {
+    Uniform& U = red.tiles->u;
+    const auto uni = uniform_pass<true>(
+        [&] {
+            const double cold = U.ref[4];
+            U.r = (cold - U.icpt) - apply_at(U.chi, dt, U.f, U.x, U.x, U.x, U.x, U.x);
+            U.cn = cold + flux_at(dt, U.f, U.x, U.x, U.x, U.x, U.x);
+            U.closure = fabs(U.cn - (U.icpt + U.chi * U.x));
+            U.mun = P.mu_ref + (U.cn - U.icpt) / U.chi;
+            const Phi3 q{U.q0, U.q1, U.q2};
+            U.bad = bad_cell<true>(P, q, U.cn, U.mun);
+            U.add[0] = U.r * U.r;
+            U.add[1] = U.cn;
+            U.add[2] = energy_cell<true>(P, q, q, q, true, U.cn, U.chi, U.icpt);
+        },
+        [&](int t, int, bool valid) {
+            if (!valid) return;
+            vclos = fmax(vclos, U.closure);
+            if (U.bad) vbad = 1;
+            const Pair c = pair_of(P, t);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const size_t i = k ? c.i1 : c.i0;
+                B.c[tr][i] = U.cn;
+                B.mu[tr][i] = U.mun;
+                vrr += U.add[0];
+                vmass += U.add[1];
+                ven += U.add[2];
+            }
+        });
+    const bool ok = sweep<9>(a, red, maps, planes, 0x3Fu, true, [&](const auto& src, const Pair& c) {
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {
             if (k == 1 && !c.v1) break;
@@ -1178,7 +1536,7 @@ __device__ bool phase_final(const Dom& a, Red& red, int cur, double dt, double& 
             vmass += cn;
             ven += energy_cell<true>(P, q, e, n, has_n, cn, chi, icpt);
         }
-    });
+    }, uni);
     if (!ok) return false;
     double v[5] = {vclos, vbad, vmass, ven, vrr};
     if (!red.reduce<5>(v, OPS5(kMax, kMax, kSum, kSum, kSum), kTagFinal)) return false;
@@ -1375,6 +1733,9 @@ __device__ bool diffusion(const Dom& a, Red& red, int cur, double dt, DiffusionO
             continue;
         }
         if (iteration == P.cg_max) break;
+        // the direction of iteration i has spread i + 1 cells into the rim; past the
+        // rim, uniform tiles are no longer uniform
+        if (red.tiles->active && iteration + 1 >= kReach && !phase_expand(a, red, pbuf)) return false;
         const int pout = pbuf ^ 1;
         double pAp;
         if (!phase_apply(a, red, dt, first, beta, pout, pAp)) return false;
@@ -1431,7 +1792,7 @@ __device__ bool advance(const Dom& a, Red& red, StepState& st, double stop_time,
         out.retries = attempt;
         out.accepted_dt = dt;
         bool mixbad, simplexbad;
-        if (!phase_propose(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
+        if (!phase_propose<!kSolve32>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
         if (simplexbad) {
             set_error(a, PEARL_ERR_SIMPLEX, 0);
             return false;
@@ -1449,6 +1810,7 @@ __device__ bool advance(const Dom& a, Red& red, StepState& st, double stop_time,
                 if (!phase_final_phase_only(a, red, st.cur, bad, e1)) return false;
             } else {
                 DiffusionOut d;
+                if (!kSolve32 && red.tiles->enabled) classify_tiles(a, *red.tiles);
                 if (!diffusion<kSolve32>(a, red, st.cur, dt, d)) return false;
                 good = d.ok;
                 out.cg_iterations = d.it;
@@ -1904,6 +2266,15 @@ __device__ void record_tape(const Dom& a, int cur, double* slot) {
         for (int f = 0; f < 6; ++f) slot[f * pe + i] = src[f][i];
 }
 
+// Whether this launch looks for uniform tiles of domain `a` (one thread).  The
+// grid's first block has the most tiles, so all blocks of the domain agree.
+__device__ __forceinline__ void init_tiles(Tiles& T, const Dom& a, bool wanted) {
+    const DevParams& P = a.P;
+    T.enabled = wanted && a.use_tma && a.B.mixed_tile && !P.phase_only && P.nty >= kMinTileRowsUniform &&
+                (P.ntiles - 1) / a.nblk + 1 <= kMaxListedTiles;
+    T.active = 0;
+}
+
 // The persistent step kernel's body; kSolve32 selects the mixed form's inner
 // solve (pearl_kernel_mixed), every other part is the same code.
 template <bool kSolve32>
@@ -1919,8 +2290,13 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
         if (threadIdx.x == 0) init_pipe(pipe);
         __syncthreads();
     }
+    __shared__ Tiles tiles;
+    // (a tape takes the whole solution plane of every step)
+    if (threadIdx.x == 0) init_tiles(tiles, a, args.mode == kModeRun && !kSolve32 && !args.tape);
+    __syncthreads();
     Red red(a, &clk);
     red.pipe_ptr = &pipe;
+    red.tiles = &tiles;
     StepState st;
     st.S = ctl->S;
     st.cur = ctl->cur;
@@ -1977,7 +2353,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     if (args.mode == kModePropose) {
         double change;
         bool mixbad, simplexbad;
-        if (!phase_propose(a, red, st.cur, args.dt, change, mixbad, simplexbad)) return;
+        if (!phase_propose<!kSolve32>(a, red, st.cur, args.dt, change, mixbad, simplexbad)) return;
         if (leader) {
             ctl->out[0] = change;
             ctl->iout[0] = mixbad;
@@ -2109,6 +2485,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
         if (threadIdx.x == 0) init_pipe(pipe);
         __syncthreads();
     }
+    __shared__ Tiles tiles;
     Ctl* gctl = args.group_ctl + g;
     double* gpart = args.group_part + (size_t)b0 * 2 * kMaxRed;
     const bool leader = bid == 0 && threadIdx.x == 0;
@@ -2122,8 +2499,11 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
         }
         __syncthreads();
         const Dom a{sP, sB, I->maps, args.use_tma, bid, nblk, gctl, gpart, 0, 0, 0, 0, 0, 0, 0};
+        if (threadIdx.x == 0) init_tiles(tiles, a, !kSolve32);
+        __syncthreads();
         Red red(a, &clk, reductions);
         red.pipe_ptr = &pipe;
+        red.tiles = &tiles;
         Ctl* ctl = sB.ctl;
         StepState st;
         st.S = ctl->S;
