@@ -264,6 +264,11 @@ struct PhaseClock {
 // are neither read nor written: 104 bytes a cell and step instead of about 950.
 // Sums keep their order and cells their arithmetic, so every result is the same
 // bit for bit; a domain without uniform tiles takes the dense path throughout.
+// Inside one launch a tile that is four or more tiles away from a non-uniform
+// one (kFar) is not even read by the next PROPOSE: what is not uniform moves by
+// less than a tile a step, so such a tile still equals the reference cell; and
+// a plane that already holds the value that a pass would write is left as it
+// is.  Both are forgotten between launches, when other calls may change planes.
 //
 // What is not uniform spreads one cell per conjugate-gradient iteration, so a
 // tile beside a non-uniform one is dense as well (the rim), and a tile beside
@@ -271,7 +276,7 @@ struct PhaseClock {
 // rim is as thick as a tile's shorter side (kReach cells): a solve that takes
 // more iterations than that writes the uniform tiles' planes and goes on dense
 // (phase_expand).  Tiles at the two walls are dense, their diagonal differs.
-enum TileClass : unsigned char { kDense = 0, kUniform = 1, kBorder = 2, kClassMask = 3, kLastColumn = 4 };
+enum TileClass : unsigned char { kDense = 0, kUniform = 1, kBorder = 2, kClassMask = 3, kLastColumn = 4, kFar = 8 };
 // Fewer tile rows leave nothing between the walls' rims and the front's.
 constexpr int kMinTileRowsUniform = 8;
 constexpr int kMaxListedTiles = 2048;  // tiles of one block; a block with more runs dense
@@ -285,17 +290,45 @@ struct Uniform {
     int have, simplex_bad, mix_bad;
     Faces f;
     double x, r, z, p, Ap, diag, cn, mun, closure;
+    bool held;  // the trial set already holds (mun, cn) in every uniform tile
     double add[3];  // the cell's contributions to the current pass's sums
     int bad;
 };
 struct Tiles {
     int enabled;  // this launch looks for uniform tiles
     int active;   // cls and list describe the current attempt
+    int known;    // the tiles marked kFar in cls are uniform in the current state
+    int skipping; // this PROPOSE leaves them out
     int ndense;
     Uniform u;
     unsigned char cls[kMaxListedTiles];    // TileClass of the block's tiles, in walk order
-    unsigned short list[kMaxListedTiles];  // positions of the dense ones
+    unsigned short list[kMaxListedTiles];  // positions of the dense (in PROPOSE: of the read) ones
+    // bit k % 32 of word k / 32: tile k is uniform, whole, and no border tile
+    unsigned plain[kMaxListedTiles / 32];
+    // bit set: the tile's phi of that state set, bit 2 + set: its mu and carbon, are
+    // all equal to content[set] (phi (3), mu, carbon)
+    unsigned char held[kMaxListedTiles];
+    double content[2][5];
+    int plain_held[2];  // every uniform and border tile of cls has bit 2 + set
 };
+__device__ __forceinline__ bool same_bits(double a, double b) {
+    return __double_as_longlong(a) == __double_as_longlong(b);
+}
+// Positions k of 0 .. nb-1 that `take` picks, in order, into T.list and T.ndense
+// (all threads; the caller synchronises the block before and after).
+template <class Take>
+__device__ __forceinline__ void list_tiles(Tiles& T, int nb, Take&& take) {
+    if (threadIdx.x >= 32) return;
+    int n = 0;
+    for (int k0 = 0; k0 < nb; k0 += 32) {
+        const int k = k0 + (int)threadIdx.x;
+        const bool dense = k < nb && take(k);
+        const unsigned votes = __ballot_sync(0xffffffffu, dense);
+        if (dense) T.list[n + __popc(votes & ((1u << threadIdx.x) - 1))] = (unsigned short)k;
+        n += __popc(votes);
+    }
+    if (threadIdx.x == 0) T.ndense = n;
+}
 
 struct Red {
     const Dom& a;
@@ -485,24 +518,50 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // a run's sums do not depend on how it is split into launches.
 // `uni` is the pass's part for uniform tiles (NoUniform: it has none): when the
 // attempt's tiles are classified, uni.prepare() runs in one thread while the
-// first copies are under way, and uni.tile(k, valid) takes the place of the
-// dense tile; `tile_end(t)` replaces the block barrier that ends a tile.
+// first copies are under way, uni.run(n) takes the place of n whole uniform
+// tiles (false: it leaves them to uni.tile), and uni.tile(pos, t, class, valid) that of the
+// tile at position pos of the block's tiles; `tile_end(t)` replaces the block barrier that ends a tile.
 struct NoUniform {
     static constexpr bool kAny = false;
+    __device__ static bool on(const Tiles&) { return false; }
     __device__ void prepare() const {}
-    __device__ void tile(int, int, bool) const {}
+    __device__ bool run(int) const { return true; }
+    __device__ void tile(int, int, int, bool) const {}
 };
-template <bool kHas, class Prepare, class Tile>
+// PROPOSE: only the listed tiles are read.
+struct ReadListed {
+    static constexpr bool kAny = true;
+    __device__ static bool on(const Tiles& T) { return T.skipping; }
+    __device__ void prepare() const {}
+    __device__ bool run(int) const { return true; }
+    __device__ void tile(int, int, int, bool) const {}
+};
+template <bool kHas, class Prepare, class Run, class Tile>
 struct UniformPass {
     static constexpr bool kAny = kHas;
     Prepare prepare_;
+    Run run_;
     Tile tile_;
+    __device__ static bool on(const Tiles& T) { return T.active; }
     __device__ void prepare() const { prepare_(); }
-    __device__ void tile(int t, int cls, bool valid) const { tile_(t, cls, valid); }
+    __device__ bool run(int n) const { return run_(n); }
+    __device__ void tile(int pos, int t, int cls, bool valid) const { tile_(pos, t, cls, valid); }
 };
-template <bool kHas, class Prepare, class Tile>
-__device__ __forceinline__ UniformPass<kHas, Prepare, Tile> uniform_pass(Prepare p, Tile t) {
-    return {p, t};
+template <bool kHas, class Prepare, class Run, class Tile>
+__device__ __forceinline__ UniformPass<kHas, Prepare, Run, Tile> uniform_pass(Prepare p, Run r, Tile t) {
+    return {p, r, t};
+}
+// A thread's running sums over n whole uniform tiles, two cells each.
+template <int NV>
+__device__ __forceinline__ void add_run(int n, const double* add, double& a, double& b, double& c) {
+    const double u = add[0], v = NV > 1 ? add[1] : 0, w = NV > 2 ? add[2] : 0;
+    for (int i = 0; i < n; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            a += u;
+            if (NV > 1) b += v;
+            if (NV > 2) c += w;
+        }
 }
 struct BlockBarrier {
     __device__ void operator()(int) const { __syncthreads(); }
@@ -542,7 +601,8 @@ __device__ bool sweep(const Dom& a, Red& red, const int (&maps)[NF], const T* co
     // read only at the cells that the reading block itself writes, after reading
     // them).  S-1 tiles ahead: the stage of tile k+S-1 is the one freed by the
     // barrier ending tile k-1.
-    const bool skip = std::remove_reference_t<Uni>::kAny && red.tiles->active;
+    using U_ = std::remove_reference_t<Uni>;
+    const bool skip = U_::kAny && U_::on(*red.tiles);
     const int nd = skip ? red.tiles->ndense : nb;  // dense tiles, staged in walk order
     const auto dense_at = [&](int d) {
         return !skip ? d : reverse ? nb - 1 - (int)red.tiles->list[nd - 1 - d] : (int)red.tiles->list[d];
@@ -566,7 +626,7 @@ __device__ bool sweep(const Dom& a, Red& red, const int (&maps)[NF], const T* co
         for (int d = 0; d < S - 1 && d < nd; ++d) issue(d);
     }
     __syncwarp();
-    if constexpr (std::remove_reference_t<Uni>::kAny) {
+    if constexpr (U_::kAny) {
         if (skip) {
             if (threadIdx.x == 32) uni.prepare();
             __syncthreads();
@@ -576,11 +636,21 @@ __device__ bool sweep(const Dom& a, Red& red, const int (&maps)[NF], const T* co
     for (int d = 0; d < nd || skip; ++d) {
         const int k = d < nd ? dense_at(d) : nb;
         if (threadIdx.x == 0 && d + S - 1 < nd) issue(d + S - 1);
-        if constexpr (std::remove_reference_t<Uni>::kAny) {
+        if constexpr (U_::kAny) {
             if (skip) {
-                for (; done < k; ++done) {
-                    const unsigned char c = red.tiles->cls[reverse ? nb - 1 - done : done];
-                    uni.tile(tile_of(done), c & kClassMask, !(c & kLastColumn) || lane < P.nx - (P.ntx - 1) * kTileX);
+                while (done < k) {
+                    const int pos = reverse ? nb - 1 - done : done;
+                    // a run of whole uniform tiles, as far as the word of marks goes
+                    const unsigned word = red.tiles->plain[pos >> 5];
+                    const int run = min(k - done, reverse ? __clz(~(word << (31 - (pos & 31))))
+                                                          : __clz(__brev(~(word >> (pos & 31)))));
+                    if (run > 0 && uni.run(run)) {
+                        done += run;
+                        continue;
+                    }
+                    const unsigned char c = red.tiles->cls[pos];
+                    ++done;
+                    uni.tile(pos, a.bid + pos * G, c & kClassMask, !(c & kLastColumn) || lane < P.nx - (P.ntx - 1) * kTileX);
                 }
                 if (d >= nd) break;
                 ++done;
@@ -774,7 +844,10 @@ __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double
     int maps[NF] = {kMapState + 5 * cur, kMapState + 5 * cur + 1, kMapState + 5 * cur + 2, kMapState + 5 * cur + 4};
     const double* planes[NF] = {B.phi[cur][0], B.phi[cur][1], B.phi[cur][2], B.mu[cur]};
     const bool find = kFindUniform && red.tiles->enabled;
-    Uniform& U = red.tiles->u;
+    Tiles& T = *red.tiles;
+    Uniform& U = T.u;
+    const int set = cur ^ 1, nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
+    bool skipping = false;  // the far tiles are known to be uniform
     bool same = true, have = false;  // this thread's cells of the tile are uniform; U holds their proposal
     if constexpr (kFindUniform) {
         maps[4] = kMapState + 5 * cur + 3;
@@ -785,14 +858,30 @@ __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double
             if (threadIdx.x < 5) U.ref[threadIdx.x] = planes[threadIdx.x][i];
             if (threadIdx.x == 0) {
                 U.have = 0;
-                red.tiles->active = 0;
+                T.active = 0;
             }
+            __syncthreads();
+            skipping = T.known;
+#pragma unroll
+            for (int f = 0; f < 5; ++f) skipping = skipping && same_bits(U.ref[f], T.content[cur][f]);
+            if (skipping) {
+                // all but the far tiles, and the first of those in the walk, whose
+                // proposal stands for the others
+                __shared__ int s_first;
+                if (threadIdx.x == 0) s_first = -1;
+                __syncthreads();
+                for (int k = threadIdx.x; k < nb; k += kThreads)
+                    if (T.cls[k] & kFar) atomicMax(&s_first, k);
+                __syncthreads();
+                list_tiles(T, nb, [&](int k) { return !(T.cls[k] & kFar) || k == s_first; });
+            }
+            if (threadIdx.x == 0) T.skipping = skipping;
             __syncthreads();
         }
     }
     const auto equals_ref = [&](const auto& src, const Pair& c) {
         if (c.y0 < kTileRows || c.y0 / kTileRows == P.nty - 1) return false;  // the tiles at the walls
-        const auto differs = [&](double v, double ref) { return __double_as_longlong(v) ^ __double_as_longlong(ref); };
+        const auto differs = [](double v, double ref) { return __double_as_longlong(v) ^ __double_as_longlong(ref); };
         long long d = differs(src.v(2, 0, kC), U.ref[2]);
         if (d) return false;
         if constexpr (kFindUniform) d = differs(src.v(4, 0, kC), U.ref[4]) | differs(src.v(4, 1, kC), U.ref[4]);
@@ -874,16 +963,50 @@ __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double
             return;
         }
         const int all = __syncthreads_and(same);
-        if (threadIdx.x == 0) B.mixed_tile[t] = !all;
+        if (threadIdx.x == 0) {
+            B.mixed_tile[t] = !all;
+            unsigned char& h = T.held[(t - a.bid) / a.nblk];
+            h = (unsigned char)((h & ~(1 << set)) | (all << set));
+        }
         same = true;  // lanes outside the domain have no say
         if (!have) have = U.have != 0;
     };
+    using Uni = std::conditional_t<kFindUniform, ReadListed, NoUniform>;
     const bool ok =
         P.mixed ? sweep<NF>(a, red, maps, planes, kWrapped, true,
-                            [&](const auto& src, const Pair& c) { body(std::true_type{}, src, c); }, NoUniform{}, tile_end)
+                            [&](const auto& src, const Pair& c) { body(std::true_type{}, src, c); }, Uni{}, tile_end)
                 : sweep<NF>(a, red, maps, planes, kWrapped, true,
-                            [&](const auto& src, const Pair& c) { body(std::false_type{}, src, c); }, NoUniform{}, tile_end);
+                            [&](const auto& src, const Pair& c) { body(std::false_type{}, src, c); }, Uni{}, tile_end);
     if (!ok) return false;
+    if (find) {
+        __syncthreads();
+        if (skipping) {
+            // the tiles left out: their proposal is U's; written where the trial set holds another
+            const bool held = same_bits(U.q0, T.content[set][0]) && same_bits(U.q1, T.content[set][1]) &&
+                              same_bits(U.q2, T.content[set][2]);
+            int missing = 0;
+            for (int k = threadIdx.x; k < nb; k += kThreads)
+                missing |= (T.cls[k] & kFar) && !((T.held[k] >> set) & 1);
+            missing = __syncthreads_or(missing);
+            int next = 0;  // T.list has the others, in order
+            for (int k = 0; k < nb && !(held && !missing); ++k) {
+                if (next < T.ndense && T.list[next] == k) {
+                    ++next;
+                    continue;
+                }
+                if (held && ((T.held[k] >> set) & 1)) continue;
+                const Pair c = pair_of(P, a.bid + k * a.nblk);
+                if (!c.v0) continue;
+                tp[0][c.i0] = tp[0][c.i1] = U.q0;
+                tp[1][c.i0] = tp[1][c.i1] = U.q1;
+                tp[2][c.i0] = tp[2][c.i1] = U.q2;
+            }
+            __syncthreads();
+            for (int k = threadIdx.x; k < nb; k += kThreads)
+                if (T.cls[k] & kFar) T.held[k] |= (unsigned char)(1 << set);
+        }
+        if (threadIdx.x < 3) T.content[set][threadIdx.x] = threadIdx.x == 0 ? U.q0 : threadIdx.x == 1 ? U.q1 : U.q2;
+    }
     double v[3] = {vchange, vmix, vsimp};
     if (!red.reduce<3>(v, OPS3(kMax, kMax, kMax), kTagPropose)) return false;
     change = v[0];
@@ -894,46 +1017,56 @@ __device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double
 
 // The classes of the block's tiles for the current attempt, from the marks that
 // PROPOSE left (all blocks', after its reduction).  A tile within one tile of a
-// marked one is dense, within two a border tile; a last column narrower than
+// marked one is dense, within two a border tile, four or more away far; a last column narrower than
 // the rim counts with the column beyond it (x is periodic).
 __device__ void classify_tiles(const Dom& a, Tiles& T) {
     const DevParams& P = a.P;
     const int nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
     const int rest = P.nx - (P.ntx - 1) * kTileX, thin = rest < kReach ? 1 : 0;
-    for (int k = threadIdx.x; k < nb; k += kThreads) {
-        const int t = a.bid + k * a.nblk, bx = t % P.ntx, by = t / P.ntx;
-        const unsigned char* m = a.B.mixed_tile;
-        int nearest = 3;
-        // all marks at once: none of the loads waits for another's outcome
+    // eight lanes a tile, one for each of the seven tile rows around it; a row's
+    // marks are read at once: none of the loads waits for another's outcome
+    const int dy = (int)(threadIdx.x & 7) - 3;
+    for (int k0 = 0; k0 < nb; k0 += kThreads / 8) {
+        const int k = k0 + (int)(threadIdx.x >> 3);
+        int nearest = 4, bx = 0;
+        if (k < nb && dy <= 3) {
+            const int t = a.bid + k * a.nblk, by = t / P.ntx;
+            bx = t - by * P.ntx;
+            // beyond a wall: the wall's own row, which is marked and nearer
+            const unsigned char* m = a.B.mixed_tile + (size_t)min(max(by + dy, 0), P.nty - 1) * P.ntx;
 #pragma unroll
-        for (int dy = -2; dy <= 2; ++dy) {
-            const int y = min(max(by + dy, 0), P.nty - 1);  // beyond a wall: the wall's own row, marked and nearer
-#pragma unroll
-            for (int dx = -3; dx <= 3; ++dx) {
+            for (int dx = -4; dx <= 4; ++dx) {
                 int x = bx + dx;
                 while (x < 0) x += P.ntx;
                 while (x >= P.ntx) x -= P.ntx;
-                const int far = max(abs(dy), max(abs(dx) - thin, 0));
-                if (m[(size_t)y * P.ntx + x]) nearest = min(nearest, far);
+                if (m[x]) nearest = min(nearest, max(abs(dy), max(abs(dx) - thin, 0)));
             }
         }
-        T.cls[k] = (unsigned char)((nearest <= 1 ? kDense : nearest == 2 ? kBorder : kUniform) |
-                                   (bx == P.ntx - 1 ? kLastColumn : 0));
+        __syncwarp();
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) nearest = min(nearest, __shfl_xor_sync(0xffffffffu, nearest, o));
+        if (k < nb && dy == -3)
+            T.cls[k] = (unsigned char)((nearest <= 1 ? kDense : nearest == 2 ? kBorder : kUniform) |
+                                       (nearest >= 4 ? kFar : 0) |
+                                       (rest < kTileX && bx == P.ntx - 1 ? kLastColumn : 0));
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        int n = 0;
+    list_tiles(T, nb, [&](int k) { return (T.cls[k] & kClassMask) == kDense; });
+    if (threadIdx.x >= 32 && threadIdx.x < 64)  // the second warp, meanwhile
         for (int k0 = 0; k0 < nb; k0 += 32) {
-            const int k = k0 + threadIdx.x;
-            const bool dense = k < nb && (T.cls[k] & kClassMask) == kDense;
-            const unsigned votes = __ballot_sync(0xffffffffu, dense);
-            if (dense) T.list[n + __popc(votes & ((1u << threadIdx.x) - 1))] = (unsigned short)k;
-            n += __popc(votes);
+            const int lane = threadIdx.x & 31;
+            const unsigned votes =
+                __ballot_sync(0xffffffffu, k0 + lane < nb && (T.cls[k0 + lane] & (kClassMask | kLastColumn)) == kUniform);
+            if (lane == 0) T.plain[k0 >> 5] = votes;
         }
-        if (threadIdx.x == 0) {
-            T.ndense = n;
-            T.active = 1;
-        }
+    int missing = 0;  // sets in which some uniform or border tile does not hold mu and carbon
+    for (int k = threadIdx.x; k < nb; k += kThreads)
+        if ((T.cls[k] & kClassMask) != kDense) missing |= ~(T.held[k] >> 2) & 3;
+    const int miss0 = __syncthreads_or(missing & 1), miss1 = __syncthreads_or(missing & 2);
+    if (threadIdx.x == 0) {
+        T.plain_held[0] = !miss0;
+        T.plain_held[1] = !miss1;
+        T.active = T.known = 1;
     }
     __syncthreads();
 }
@@ -988,7 +1121,11 @@ __device__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& 
             U.add[1] = U.r * U.z;
             U.add[2] = U.r * U.r;
         },
-        [&](int t, int cls, bool valid) {
+        [&](int n) {
+            add_run<3>(n, U.add, s0, s1, s2);
+            return true;
+        },
+        [&](int, int t, int cls, bool valid) {
             if (!valid) return;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -1101,7 +1238,11 @@ __device__ bool phase_apply(const Dom& a, Red& red, double dt, bool first, doubl
             U.Ap = apply_at(U.chi, dt, U.f, U.p, U.p, U.p, U.p, U.p);
             U.add[0] = U.p * U.Ap;
         },
-        [&](int t, int cls, bool valid) {
+        [&](int n) {
+            add_run<1>(n, U.add, s, s, s);
+            return true;
+        },
+        [&](int, int t, int cls, bool valid) {
             if (!valid) return;
             s += U.add[0];
             s += U.add[0];
@@ -1143,7 +1284,11 @@ __device__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, dou
             U.add[0] = U.r * U.z;
             U.add[1] = U.r * U.r;
         },
-        [&](int t, int cls, bool valid) {
+        [&](int n) {
+            add_run<2>(n, U.add, s0, s1, s1);
+            return true;
+        },
+        [&](int, int t, int cls, bool valid) {
             if (!valid) return;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -1227,6 +1372,8 @@ __device__ bool phase_expand(const Dom& a, Red& red, int pcur) {
         for (int k = 0; k < 2; ++k) {
             if (!(k ? c.v1 : c.v0)) continue;
             const size_t i = k ? c.i1 : c.i0;
+            B.chi[i] = U.chi;
+            B.icpt[i] = U.icpt;
             B.wE[i] = U.f.w1;
             B.wN[i] = U.f.w3;
             B.diag[i] = U.diag;
@@ -1238,7 +1385,7 @@ __device__ bool phase_expand(const Dom& a, Red& red, int pcur) {
     }
     double v[1] = {0};
     if (!red.reduce<1>(v, kMax, kTagReset)) return false;
-    if (threadIdx.x == 0) red.tiles->active = 0;
+    if (threadIdx.x == 0) red.tiles->active = red.tiles->known = 0;
     __syncthreads();
     return true;
 }
@@ -1490,23 +1637,36 @@ __device__ bool phase_final(const Dom& a, Red& red, int cur, double dt, double& 
             U.mun = P.mu_ref + (U.cn - U.icpt) / U.chi;
             const Phi3 q{U.q0, U.q1, U.q2};
             U.bad = bad_cell<true>(P, q, U.cn, U.mun);
+            U.held = red.tiles->plain_held[tr] && same_bits(U.mun, red.tiles->content[tr][3]) &&
+                     same_bits(U.cn, red.tiles->content[tr][4]);
             U.add[0] = U.r * U.r;
             U.add[1] = U.cn;
             U.add[2] = energy_cell<true>(P, q, q, q, true, U.cn, U.chi, U.icpt);
         },
-        [&](int t, int, bool valid) {
+        [&](int n) {
+            if (!U.held) return false;
+            vclos = fmax(vclos, U.closure);
+            if (U.bad) vbad = 1;
+            add_run<3>(n, U.add, vrr, vmass, ven);
+            return true;
+        },
+        [&](int pos, int t, int, bool valid) {
             if (!valid) return;
             vclos = fmax(vclos, U.closure);
             if (U.bad) vbad = 1;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                vrr += U.add[0];
+                vmass += U.add[1];
+                ven += U.add[2];
+            }
+            if (U.held) return;
             const Pair c = pair_of(P, t);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const size_t i = k ? c.i1 : c.i0;
                 B.c[tr][i] = U.cn;
                 B.mu[tr][i] = U.mun;
-                vrr += U.add[0];
-                vmass += U.add[1];
-                ven += U.add[2];
             }
         });
     const bool ok = sweep<9>(a, red, maps, planes, 0x3Fu, true, [&](const auto& src, const Pair& c) {
@@ -1540,6 +1700,16 @@ __device__ bool phase_final(const Dom& a, Red& red, int cur, double dt, double& 
     if (!ok) return false;
     double v[5] = {vclos, vbad, vmass, ven, vrr};
     if (!red.reduce<5>(v, OPS5(kMax, kMax, kSum, kSum, kSum), kTagFinal)) return false;
+    if (red.tiles->enabled) {
+        Tiles& T = *red.tiles;
+        const int nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
+        for (int k = threadIdx.x; k < nb; k += kThreads) {
+            const bool uniform = T.active && (T.cls[k] & kClassMask) != kDense;
+            T.held[k] = (unsigned char)((T.held[k] & ~(4 << tr)) | (uniform ? 4 << tr : 0));
+        }
+        if (threadIdx.x < 2) T.content[tr][3 + threadIdx.x] = threadIdx.x ? U.cn : U.mun;
+        __syncthreads();
+    }
     closure = v[0];
     bad = v[1] != 0;
     mass = v[2] * P.dx * P.dy;
@@ -1843,6 +2013,12 @@ __device__ bool advance(const Dom& a, Red& red, StepState& st, double stop_time,
             const double grown = dt * 1.1;
             st.S.dt = grown < P.dt_max ? grown : P.dt_max;
             st.cur ^= 1;
+            // after more iterations than this what is not uniform may have moved by a tile
+            if (red.tiles->known && out.cg_iterations + 1 >= kReach) {
+                __syncthreads();
+                if (threadIdx.x == 0) red.tiles->known = 0;
+                __syncthreads();
+            }
             st.e0 = P.check_energy ? e1 : 0;
             st.mass0 = P.phase_only ? 0 : mass;
             info = out;
@@ -2266,13 +2442,20 @@ __device__ void record_tape(const Dom& a, int cur, double* slot) {
         for (int f = 0; f < 6; ++f) slot[f * pe + i] = src[f][i];
 }
 
-// Whether this launch looks for uniform tiles of domain `a` (one thread).  The
-// grid's first block has the most tiles, so all blocks of the domain agree.
+// Whether this launch looks for uniform tiles of domain `a` (all threads; the
+// caller synchronises after).  The grid's first block has the most tiles, so
+// all blocks of the domain agree.
 __device__ __forceinline__ void init_tiles(Tiles& T, const Dom& a, bool wanted) {
     const DevParams& P = a.P;
-    T.enabled = wanted && a.use_tma && a.B.mixed_tile && !P.phase_only && P.nty >= kMinTileRowsUniform &&
-                (P.ntiles - 1) / a.nblk + 1 <= kMaxListedTiles;
-    T.active = 0;
+    const int most = (P.ntiles - 1) / a.nblk + 1;
+    const bool enabled = wanted && a.use_tma && a.B.mixed_tile && !P.phase_only && P.nty >= kMinTileRowsUniform &&
+                         most <= kMaxListedTiles;
+    if (threadIdx.x == 0) {
+        T.enabled = enabled;
+        T.active = T.known = T.skipping = 0;
+    }
+    if (enabled)
+        for (int k = threadIdx.x; k < most; k += kThreads) T.held[k] = 0;
 }
 
 // The persistent step kernel's body; kSolve32 selects the mixed form's inner
@@ -2292,7 +2475,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     }
     __shared__ Tiles tiles;
     // (a tape takes the whole solution plane of every step)
-    if (threadIdx.x == 0) init_tiles(tiles, a, args.mode == kModeRun && !kSolve32 && !args.tape);
+    init_tiles(tiles, a, args.mode == kModeRun && !kSolve32 && !args.tape);
     __syncthreads();
     Red red(a, &clk);
     red.pipe_ptr = &pipe;
@@ -2499,7 +2682,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
         }
         __syncthreads();
         const Dom a{sP, sB, I->maps, args.use_tma, bid, nblk, gctl, gpart, 0, 0, 0, 0, 0, 0, 0};
-        if (threadIdx.x == 0) init_tiles(tiles, a, !kSolve32);
+        init_tiles(tiles, a, !kSolve32);
         __syncthreads();
         Red red(a, &clk, reductions);
         red.pipe_ptr = &pipe;
