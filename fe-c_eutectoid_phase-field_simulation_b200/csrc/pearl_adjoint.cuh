@@ -54,19 +54,20 @@ __device__ __forceinline__ void adj_forces(const DevParams& P, const double q[3]
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const double dh = dtr[aa] + (b == aa ? 6.0 * q[b] * (1.0 - q[b]) : 0.0);
-            f[aa] += div_by(P, (ps[b] - psi0) * dh, P.Vm, P.r_Vm);
+            f[aa] += div_const(P, (ps[b] - psi0) * dh, P.Vm, P.r_Vm, P.l_Vm);
         }
     }
 #pragma unroll
     for (int dir = 0; dir < 4; ++dir) {
         if (!has[dir]) continue;
         const double* n = nb[dir];
-        const double d2 = dir < 2 ? P.dx2 : P.dy2, rd2 = dir < 2 ? P.r_dx2 : P.r_dy2;
+        const double d2 = dir < 2 ? P.dx2 : P.dy2;
+        const double rd2 = dir < 2 ? P.r_dx2 : P.r_dy2, ld2 = dir < 2 ? P.l_dx2 : P.l_dy2;
 #pragma unroll
         for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
             for (int b = aa + 1; b < 3; ++b) {
-                const double w = div_by(P, P.two_eps_sigma * (q[aa] * n[b] - n[aa] * q[b]), d2, rd2);
+                const double w = div_const(P, P.two_eps_sigma * (q[aa] * n[b] - n[aa] * q[b]), d2, rd2, ld2);
                 f[aa] += w * n[b];
                 f[b] -= w * n[aa];
             }
@@ -246,7 +247,7 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
         const double m = s0[4 * pe + i];
         double f[3];
         adj_forces(P, q, m, nb, c.has, f);
-        const double mean = div_by(P, f[0] + f[1] + f[2], 3.0, P.r_3);
+        const double mean = div_const(P, f[0] + f[1] + f[2], 3.0, P.r_3, P.l_3);
         const double tau = local_tau(P, q[0], q[1], q[2]);
         const double sc = dt / (tau * P.eps);
         double gg[3], z[3];

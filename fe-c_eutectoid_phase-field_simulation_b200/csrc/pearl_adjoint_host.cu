@@ -24,10 +24,11 @@ constexpr int kAdjThreads = tile_geometry(8).threads;
 
 int launch_adjoint(pearl_gpu_ctx* ctx, AdjArgs& args) {
     const NvtxRange range(args.mode == 0 ? "pearl_gpu adjoint seed" : "pearl_gpu adjoint segment");
+    const void* const kernel = ctx->P.fast_div ? (const void*)g8::pearl_adjoint_kernel : (const void*)g8_div::pearl_adjoint_kernel;
     if (!ctx->adj_grid) {
         int per_sm = 0, sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, g8::pearl_adjoint_kernel, kAdjThreads, 0));
+        PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kAdjThreads, 0));
         if (per_sm < 1) return fail(ctx, PEARL_ERR_CUDA, "adjoint kernel cannot be resident");
         const long long cells = (long long)ctx->nx * ctx->ny;
         const long long want = (cells + kAdjThreads - 1) / kAdjThreads;
@@ -42,7 +43,7 @@ int launch_adjoint(pearl_gpu_ctx* ctx, AdjArgs& args) {
     args.P = ctx->P;
     args.B = ctx->B;
     void* kargs[] = {&args};
-    PG_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)g8::pearl_adjoint_kernel, dim3(ctx->adj_grid), dim3(kAdjThreads),
+    PG_CUDA(ctx, cudaLaunchCooperativeKernel(kernel, dim3(ctx->adj_grid), dim3(kAdjThreads),
                                              kargs, 0, ctx->stream));
     ctx->launches++;
     rc = pull_ctl(ctx);

@@ -228,6 +228,13 @@ int batch_configure(pearl_gpu_batch* b, int gb, bool use_tma, int wx) {
     return PEARL_OK;
 }
 
+const void* batch_kernel(bool solve32, bool fast_div) {
+    static const void* const kernels[2][2] = {
+        {(const void*)g8_div::pearl_batch_kernel, (const void*)g8::pearl_batch_kernel},
+        {(const void*)g8_div::pearl_batch_kernel_mixed, (const void*)g8::pearl_batch_kernel_mixed}};
+    return kernels[solve32][fast_div];
+}
+
 int batch_launch(pearl_gpu_batch* b, const pearl_run_limits& L) {
     const NvtxRange range("pearl_gpu batch run");
     PB_CUDA(b, cudaSetDevice(b->device));
@@ -249,7 +256,10 @@ int batch_launch(pearl_gpu_batch* b, const pearl_run_limits& L) {
     // of a batch share one precision, pearl_gpu_batch_set_precision)
     bool solve32 = false;
     for (auto* c : b->inst) solve32 = solve32 || c->P.mixed_cg;
-    const void* kernel = solve32 ? (const void*)g8::pearl_batch_kernel_mixed : (const void*)g8::pearl_batch_kernel;
+    // one instance whose divisors need the general division decides for all
+    bool fast = true;
+    for (auto* c : b->inst) fast = fast && c->P.fast_div;
+    const void* kernel = batch_kernel(solve32, fast);
     PB_CUDA(b, cudaLaunchCooperativeKernel(kernel, dim3(b->grid), dim3(g.threads), kargs,
                                            b->use_tma ? g.tma_smem_bytes : 0, b->stream));
     b->launches++;
@@ -323,7 +333,8 @@ int pearl_gpu_batch_create(int n, const pearl_params* params, const int* nx, con
     if (cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess)
         return bail(PEARL_ERR_CUDA);
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device);
-    const void* kernels[2] = {(const void*)g8::pearl_batch_kernel, (const void*)g8::pearl_batch_kernel_mixed};
+    const void* kernels[4];
+    for (int k = 0; k < 4; ++k) kernels[k] = batch_kernel(k & 1, k & 2);
     for (const void* k : kernels)
         if (tma && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)tile_geometry(8).tma_smem_bytes) != cudaSuccess)

@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "pearl_division.hpp"
 #include "pearl_host.hpp"
 
 using namespace pearl_gpu;
@@ -73,9 +74,15 @@ void set_tile_shape(pearl_gpu_ctx* ctx, int wx_log2) {
     P.ntiles = P.ntx * P.nty;
 }
 
-const void* step_kernel(int warps, bool solve32) {
-    if (solve32) return warps == 16 ? (const void*)g16::pearl_kernel_mixed : (const void*)g8::pearl_kernel_mixed;
-    return warps == 16 ? (const void*)g16::pearl_kernel : (const void*)g8::pearl_kernel;
+const void* step_kernel(int warps, StepKernel kind, bool fast_div) {
+    static const void* const kernels[2][3][2] = {
+        {{(const void*)g8_div::pearl_kernel, (const void*)g8::pearl_kernel},
+         {(const void*)g8_div::pearl_kernel_mixed, (const void*)g8::pearl_kernel_mixed},
+         {(const void*)g8_div::pearl_kernel_modes, (const void*)g8::pearl_kernel_modes}},
+        {{(const void*)g16_div::pearl_kernel, (const void*)g16::pearl_kernel},
+         {(const void*)g16_div::pearl_kernel_mixed, (const void*)g16::pearl_kernel_mixed},
+         {(const void*)g16_div::pearl_kernel_modes, (const void*)g16::pearl_kernel_modes}}};
+    return kernels[warps == 16][kind][fast_div];
 }
 
 void set_geometry(pearl_gpu_ctx* ctx, int warps) {
@@ -156,19 +163,20 @@ void fill_dev_params(pearl_gpu_ctx* ctx) {
     P.max_retries = p->max_retries;
     P.check_energy = p->check_energy;
     P.phase_only = p->phase_only;
-    // reciprocals of the constant divisors (RN(1/b), host IEEE division)
-    P.r_Vm = 1.0 / P.Vm;
-    P.r_dx = 1.0 / P.dx;
-    P.r_dy = 1.0 / P.dy;
-    P.r_dx2 = 1.0 / P.dx2;
-    P.r_dy2 = 1.0 / P.dy2;
-    P.r_3 = 1.0 / 3.0;
-    for (int i = 0; i < 3; ++i) P.r_two_A[i] = 1.0 / P.two_A[i];
-    const double divisors[] = {P.Vm, P.dx, P.dy, P.dx2, P.dy2, 3.0, P.two_A[0], P.two_A[1], P.two_A[2]};
-    const double recips[] = {P.r_Vm, P.r_dx, P.r_dy, P.r_dx2, P.r_dy2, P.r_3, P.r_two_A[0], P.r_two_A[1], P.r_two_A[2]};
-    P.exact_div = 1;
-    for (int i = 0; i < 9; ++i)
-        if (std::fpclassify(divisors[i]) != FP_NORMAL || std::fpclassify(recips[i]) != FP_NORMAL) P.exact_div = 0;
+    // constants of the divisions by Vm, dx, dy, dx^2, dy^2, 3 and 2A
+    struct {
+        double b;
+        double *zh, *zl;
+    } const divisors[] = {{P.Vm, &P.r_Vm, &P.l_Vm},    {P.dx, &P.r_dx, &P.l_dx},    {P.dy, &P.r_dy, &P.l_dy},
+                          {P.dx2, &P.r_dx2, &P.l_dx2}, {P.dy2, &P.r_dy2, &P.l_dy2}, {3.0, &P.r_3, &P.l_3},
+                          {P.two_A[0], &P.r_two_A[0], &P.l_two_A[0]},
+                          {P.two_A[1], &P.r_two_A[1], &P.l_two_A[1]},
+                          {P.two_A[2], &P.r_two_A[2], &P.l_two_A[2]}};
+    P.exact_div = P.fast_div = 1;
+    for (const auto& d : divisors) {
+        if (!exact_reciprocal(d.b, *d.zh, *d.zl)) P.fast_div = 0;
+        if (std::fpclassify(d.b) != FP_NORMAL || std::fpclassify(*d.zh) != FP_NORMAL) P.exact_div = 0;
+    }
 }
 
 int pull_ctl(pearl_gpu_ctx* ctx) {
@@ -204,9 +212,9 @@ int launch(pearl_gpu_ctx* ctx, KArgs& args) {
     args.use_tma = tma ? 1 : 0;
     if (tma) std::memcpy(args.maps, ctx->maps, sizeof ctx->maps);
     const TileGeometry g = tile_geometry(ctx->warps);
-    // the mixed-solve kernel holds only the run mode
-    const bool solve32 = ctx->P.mixed_cg != 0 && args.mode == kModeRun;
-    PG_CUDA(ctx, cudaLaunchCooperativeKernel(step_kernel(ctx->warps, solve32), dim3(ctx->grid),
+    const StepKernel kind = args.mode != kModeRun ? kStepModes : ctx->P.mixed_cg ? kStepRunMixed : kStepRun;
+    PG_CUDA(ctx, cudaLaunchCooperativeKernel(step_kernel(ctx->warps, kind, ctx->P.fast_div != 0),
+                                             dim3(ctx->grid),
                                              dim3(g.threads), kargs,
                                              tma ? g.tma_smem_bytes : 0, ctx->stream));
     ctx->launches++;
@@ -618,17 +626,19 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     const char* tma_env = std::getenv("PEARL_GPU_TMA");
     ctx->use_tma = ctx->P.warps_x_log2 == 0 && !(tma_env && std::atoi(tma_env) == 0);
     const TileGeometry geom = tile_geometry(ctx->warps);
-    // both the FP64 kernel and the mixed-solve kernel of the block shape get the
-    // stage buffers; the grid fits the residency of both
-    for (bool solve32 : {false, true})
-        if (ctx->use_tma && cudaFuncSetAttribute(step_kernel(ctx->warps, solve32),
+    // every kernel of the block shape (parameters and precision may change later)
+    // gets the stage buffers; the grid fits the residency of all
+    const void* kernels[6];
+    for (int k = 0; k < 6; ++k) kernels[k] = step_kernel(ctx->warps, (StepKernel)(k / 2), k & 1);
+    for (const void* k : kernels)
+        if (ctx->use_tma && cudaFuncSetAttribute(k,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)geom.tma_smem_bytes) != cudaSuccess)
             ctx->use_tma = false;
     int per_sm = 1 << 30;
-    for (bool solve32 : {false, true}) {
+    for (const void* k : kernels) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel(ctx->warps, solve32), geom.threads,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, geom.threads,
                                                           ctx->use_tma ? geom.tma_smem_bytes : 0) != cudaSuccess ||
             n < 1)
             return bail(PEARL_ERR_CUDA);

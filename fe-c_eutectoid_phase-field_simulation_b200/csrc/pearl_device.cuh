@@ -15,6 +15,27 @@
 
 #include "pearl_gpu.h"
 
+// The device code is compiled for two block shapes (PEARL_TILE_WARPS) and two
+// ways of dividing by the formulas' constants (PEARL_FAST_DIV, see div_const),
+// each in a namespace of its own.
+#ifndef PEARL_TILE_WARPS
+#define PEARL_TILE_WARPS 8
+#endif
+#ifndef PEARL_FAST_DIV
+#define PEARL_FAST_DIV 1
+#endif
+#if PEARL_TILE_WARPS == 16
+#define PEARL_GEOM_NS PEARL_NS_(g16, PEARL_FAST_DIV)
+#elif PEARL_TILE_WARPS == 8
+#define PEARL_GEOM_NS PEARL_NS_(g8, PEARL_FAST_DIV)
+#else
+#error "PEARL_TILE_WARPS must be 8 or 16"
+#endif
+#define PEARL_NS_(g, f) PEARL_NS2_(g, f)
+#define PEARL_NS2_(g, f) PEARL_NS##f##_(g)
+#define PEARL_NS1_(g) g
+#define PEARL_NS0_(g) g##_div  // general division
+
 namespace pearl_gpu {
 
 constexpr int kTileX = 32;  // one warp spans 32 consecutive x cells (256 B of a row)
@@ -39,9 +60,11 @@ struct DevParams {
     double mass_scale;    // gx*gy*dx*dy*1e-6                  (:1152)
     double energy_scale;  // sigma*max(gx*dx, gy*dy)            (:1157)
     int cg_max, max_retries, check_energy, phase_only;
-    // RN(1/b) of every constant divisor b, for div_by
+    // RN(1/b) of every constant divisor b, for div_by, and its correction, for div_const
     double r_Vm, r_dx, r_dy, r_dx2, r_dy2, r_3, r_two_A[3];
+    double l_Vm, l_dx, l_dy, l_dx2, l_dy2, l_3, l_two_A[3];
     int exact_div;  // 1 when every constant divisor and its reciprocal are normal numbers
+    int fast_div;   // 1 when exact_reciprocal found the correction of every divisor
     // Mixed precision (PROPOSE forces in FP32).  psi_b(mu) - psi_g(mu) is
     // expanded about mu_ref in delta = mu - mu_ref, which is formed in FP64:
     // m_pa[b] + delta*(m_pb[b] + delta*m_pc[b]), so FP32 never subtracts two
@@ -72,8 +95,7 @@ struct DevParams {
 // The zero / non-finite test reads the bit patterns with integer operations,
 // which leaves the FP64 pipe to the arithmetic: a == +-0 when its magnitude
 // bits are all zero, q0 is Inf or NaN when its exponent field is all ones.
-__device__ __forceinline__ double div_by(const DevParams& P, double a, double b, double rb) {
-    if (!P.exact_div) return a / b;
+__device__ __forceinline__ double div_corrected(double a, double b, double rb) {
     const double q0 = a * rb;
     double r = fma(-q0, b, a);
     double q = fma(r, rb, q0);
@@ -83,24 +105,29 @@ __device__ __forceinline__ double div_by(const DevParams& P, double a, double b,
     const bool special = (((ah & 0x7fffffff) | al) == 0) | ((qh & 0x7ff00000) == 0x7ff00000);
     return special ? q0 : q;
 }
-
-// div_by for the proposal's forces (positive divisors only): the same
-// correctly rounded quotient for finite numerators and quotients, but without
-// div_by's integer tests.  A zero numerator's sign is OR-ed into the result
-// (the corrections turn -0 into +0, and a nonzero quotient already has the
-// numerator's sign); a non-finite numerator gives NaN where IEEE division
-// gives +-Inf.  Both are non-finite, and the proposal treats any non-finite
-// force alike: the cell takes the reference's non-finite branch
-// (pearl_serial.cpp:990-996), keeps its phi and reports an infinite change.
-__device__ __forceinline__ double div_force(const DevParams& P, double a, double b, double rb) {
-    if (!P.exact_div) return a / b;
-    const double q0 = a * rb;
-    double r = fma(-q0, b, a);
-    double q = fma(r, rb, q0);
-    r = fma(-q, b, a);
-    q = fma(r, rb, q);
-    return __hiloint2double(__double2hiint(q) | (__double2hiint(a) & (int)0x80000000), __double2loint(q));
+__device__ __forceinline__ double div_by(const DevParams& P, double a, double b, double rb) {
+    return P.exact_div ? div_corrected(a, b, rb) : a / b;
 }
+
+namespace PEARL_GEOM_NS {
+// a/b, correctly rounded, for a divisor with constants zh and zl that
+// exact_reciprocal has proved right for every normal numerator: two dependent
+// FP64 operations where div_by takes five and its integer tests (PROPOSE has 20
+// of these divisions a cell, FINAL 10, and both are bound by FP64 issue and
+// latency).  The sign of a zero numerator may be lost and a non-finite
+// numerator gives some non-finite value: no force, face weight or energy
+// depends on either.  (A force's terms are added to a sum that is never -0, and
+// a non-finite force sends the cell down the reference's non-finite branch,
+// pearl_serial.cpp:990-996, whatever its value; an energy squares its
+// quotients, and a non-finite trial fails valid_state first.)  The kernels of
+// the general namespaces, for the one parameter set in a hundred with a divisor
+// that exact_reciprocal refuses, divide with div_by: a choice inside one kernel
+// puts a branch at every quotient, which held PROPOSE at 183 us on 2048x4096.
+__device__ __forceinline__ double div_const(const DevParams& P, double a, double b, double zh, double zl) {
+    if constexpr (PEARL_FAST_DIV != 0) return fma(a, zh, a * zl);
+    return div_by(P, a, b, zh);
+}
+}  // namespace PEARL_GEOM_NS
 
 // Device buffers: two state sets (current / trial, selected by Ctl::cur) and
 // the work vectors of the implicit solve.  Every plane is ny rows of `pitch`
@@ -194,10 +221,11 @@ __device__ __forceinline__ bool mixture(const DevParams& P, double p0, double p1
     return (s > 0.0) && isfinite(s) && isfinite(ci) && isfinite(k) && !(k < 0.0);
 }
 
+namespace PEARL_GEOM_NS {
 // project_simplex (pearl_serial.cpp:491-509).  Inputs are finite here (the
 // caller checks first, :990-996).  Returns false where the reference throws.
 // The thresholds (sum-1)/1, /2, /3 are formed exactly: x/1 = x, x/2 = x*0.5,
-// and /3 through div_by.
+// and /3 through div_const.
 __device__ __forceinline__ bool project_simplex(const DevParams& P, double& z0, double& z1, double& z2) {
     double s0 = z0, s1 = z1, s2 = z2, t;
     if (s0 < s1) { t = s0; s0 = s1; s1 = t; }
@@ -212,7 +240,7 @@ __device__ __forceinline__ bool project_simplex(const DevParams& P, double& z0, 
     cand = (sum - 1.0) * 0.5;
     if (s1 > cand) { active = 2; threshold = cand; }
     sum += s2;
-    cand = div_by(P, sum - 1.0, 3.0, P.r_3);
+    cand = div_const(P, sum - 1.0, 3.0, P.r_3, P.l_3);
     if (s2 > cand) { active = 3; threshold = cand; }
     // std::max(0.0, v) == (0.0 < v ? v : 0.0)
     double v = z0 - threshold;
@@ -223,6 +251,7 @@ __device__ __forceinline__ bool project_simplex(const DevParams& P, double& z0, 
     z2 = (0.0 < v) ? v : 0.0;
     return active != 0;
 }
+}  // namespace PEARL_GEOM_NS
 
 // local_tau (pearl_serial.cpp:533-537)
 __device__ __forceinline__ double local_tau(const DevParams& P, double p0, double p1, double p2) {
@@ -267,17 +296,6 @@ constexpr TileGeometry tile_geometry(int warps) {
     return TileGeometry{warps, 32 * warps, 2 * warps, box_h, stride, pipe, 128 + pipe * sizeof(double),
                         warps >= 16 ? 1 : 2};
 }
-
-#ifndef PEARL_TILE_WARPS
-#define PEARL_TILE_WARPS 8
-#endif
-#if PEARL_TILE_WARPS == 16
-#define PEARL_GEOM_NS g16
-#elif PEARL_TILE_WARPS == 8
-#define PEARL_GEOM_NS g8
-#else
-#error "PEARL_TILE_WARPS must be 8 or 16"
-#endif
 
 // The block shape this translation unit's device code is compiled for.
 namespace PEARL_GEOM_NS {

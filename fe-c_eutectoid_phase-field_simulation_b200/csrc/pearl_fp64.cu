@@ -128,12 +128,12 @@ struct Faces {
     double w0, w1, w2, w3;
 };
 // K is finite and nonnegative here (SET-UP runs only on a trial whose mixture
-// passed its checks, pearl_serial.cpp:136), so div_force gives div_by's bits.
+// passed its checks, pearl_serial.cpp:136), so div_const gives IEEE division's bits.
 __device__ __forceinline__ double face_x(const DevParams& P, double k, double kn) {
-    return div_force(P, .5 * (k + kn), P.dx2, P.r_dx2);
+    return div_const(P, .5 * (k + kn), P.dx2, P.r_dx2, P.l_dx2);
 }
 __device__ __forceinline__ double face_y(const DevParams& P, double k, double kn) {
-    return div_force(P, .5 * (k + kn), P.dy2, P.r_dy2);
+    return div_const(P, .5 * (k + kn), P.dy2, P.r_dy2, P.l_dy2);
 }
 __device__ __forceinline__ Faces faces0(const DevParams& P, const S2& K, const Pair& c) {
     Faces f;
@@ -178,9 +178,9 @@ __device__ __forceinline__ double flux_at(double dt, const Faces& f, double u, d
 struct Phi3 {
     double a, t, g;
 };
-#define DIVC(P, a, b, rb) (kForce ? div_force(P, a, b, rb) : div_by(P, a, b, rb))
+#define DIVC(P, a, b, rb, lb) (kForce ? div_const(P, a, b, rb, lb) : div_by(P, a, b, rb))
 // kForce: the final update's evaluation, whose divisions skip div_by's
-// operand tests (div_force): the same value for a finite state, and a state
+// operand tests (div_const): the same value for a finite state, and a state
 // that is not finite is rejected by valid_state before its energy is looked at.
 template <bool kForce = false>
 __device__ __forceinline__ double energy_cell(const DevParams& P, const Phi3& q, const Phi3& e, const Phi3& n,
@@ -197,19 +197,19 @@ __device__ __forceinline__ double energy_cell(const DevParams& P, const Phi3& q,
         const double dc = carbon - icpt;
         chem += .5 * dc * dc / chi;
     }
-    double t = DIVC(P, chem, P.Vm, P.r_Vm) + P.obs * (q.a * q.t + q.a * q.g + q.t * q.g) + P.tr * q.a * q.t * q.g;
-    double z = DIVC(P, q.a * e.t - e.a * q.t, P.dx, P.r_dx);
+    double t = DIVC(P, chem, P.Vm, P.r_Vm, P.l_Vm) + P.obs * (q.a * q.t + q.a * q.g + q.t * q.g) + P.tr * q.a * q.t * q.g;
+    double z = DIVC(P, q.a * e.t - e.a * q.t, P.dx, P.r_dx, P.l_dx);
     t += P.eps_sigma * z * z;
-    z = DIVC(P, q.a * e.g - e.a * q.g, P.dx, P.r_dx);
+    z = DIVC(P, q.a * e.g - e.a * q.g, P.dx, P.r_dx, P.l_dx);
     t += P.eps_sigma * z * z;
-    z = DIVC(P, q.t * e.g - e.t * q.g, P.dx, P.r_dx);
+    z = DIVC(P, q.t * e.g - e.t * q.g, P.dx, P.r_dx, P.l_dx);
     t += P.eps_sigma * z * z;
     if (has_n) {
-        z = DIVC(P, q.a * n.t - n.a * q.t, P.dy, P.r_dy);
+        z = DIVC(P, q.a * n.t - n.a * q.t, P.dy, P.r_dy, P.l_dy);
         t += P.eps_sigma * z * z;
-        z = DIVC(P, q.a * n.g - n.a * q.g, P.dy, P.r_dy);
+        z = DIVC(P, q.a * n.g - n.a * q.g, P.dy, P.r_dy, P.l_dy);
         t += P.eps_sigma * z * z;
-        z = DIVC(P, q.t * n.g - n.t * q.g, P.dy, P.r_dy);
+        z = DIVC(P, q.t * n.g - n.t * q.g, P.dy, P.r_dy, P.l_dy);
         t += P.eps_sigma * z * z;
     }
     return t;
@@ -235,7 +235,7 @@ __device__ __forceinline__ bool bad_cell(const DevParams& P, const Phi3& q, doub
 #pragma unroll
         for (int a = 0; a < 3; ++a)
             if (qq[a] > .01) {
-                const double ca = DIVC(P, mu - P.B[a], P.two_A[a], P.r_two_A[a]);
+                const double ca = DIVC(P, mu - P.B[a], P.two_A[a], P.r_two_A[a], P.l_two_A[a]);
                 good = good && ca >= -1e-10 && ca <= 1 + 1e-10;
             }
     }
@@ -349,7 +349,7 @@ struct Red {
     __device__ bool keeps_clock() const { return a.bid == 0 && threadIdx.x == 32; }
     // publish the block partials, wait for the grid, combine; false on a device-wait timeout
     template <int NV>
-    __device__ bool reduce(double (&v)[NV], unsigned ops, int tag) {
+    __device__ __forceinline__ bool reduce(double (&v)[NV], unsigned ops, int tag) {
         // this thread's plane stores may be read by TMA (async proxy) after the barrier
         if (a.use_tma) fence_proxy_async();
         double* slot = a.part + (size_t)(counter & 1u) * a.nblk * kMaxRed;
@@ -567,7 +567,7 @@ struct BlockBarrier {
     __device__ void operator()(int) const { __syncthreads(); }
 };
 template <int NF, bool kTileOnly = false, class T = double, class Body, class Uni = NoUniform, class End = BlockBarrier>
-__device__ bool sweep(const Dom& a, Red& red, const int (&maps)[NF], const T* const (&planes)[NF],
+__device__ __forceinline__ bool sweep(const Dom& a, Red& red, const int (&maps)[NF], const T* const (&planes)[NF],
                       unsigned stencil, bool reverse, Body&& body, Uni&& uni = Uni{}, End&& tile_end = End{}) {
     Pipe& pp = *red.pipe_ptr;
     using G_ = StageGeom<T>;
@@ -726,7 +726,7 @@ __device__ __forceinline__ Proposal propose_cell(const DevParams& P, const Src& 
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const double dh = dtr[aa] + (b == aa ? 6.0 * q[b] * (1.0 - q[b]) : 0.0);
-            f[aa] += div_force(P, (ps[b] - psi0) * dh, P.Vm, P.r_Vm);
+            f[aa] += div_const(P, (ps[b] - psi0) * dh, P.Vm, P.r_Vm, P.l_Vm);
         }
     }
     // four faces in the reference's order: -x, +x, -y (not at y=0), +y (not at the top)
@@ -735,17 +735,18 @@ __device__ __forceinline__ Proposal propose_cell(const DevParams& P, const Src& 
         if ((dir == 2 && !south) || (dir == 3 && !north)) continue;
         const int d = dir == 0 ? kW : dir == 1 ? kE : dir == 2 ? kS : kN;
         const double n[3] = {src.v(0, k, d), src.v(1, k, d), src.v(2, k, d)};
-        const double d2 = dir < 2 ? P.dx2 : P.dy2, rd2 = dir < 2 ? P.r_dx2 : P.r_dy2;
+        const double d2 = dir < 2 ? P.dx2 : P.dy2;
+        const double rd2 = dir < 2 ? P.r_dx2 : P.r_dy2, ld2 = dir < 2 ? P.l_dx2 : P.l_dy2;
 #pragma unroll
         for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
             for (int b = aa + 1; b < 3; ++b) {
-                const double w = div_force(P, P.two_eps_sigma * (q[aa] * n[b] - n[aa] * q[b]), d2, rd2);
+                const double w = div_const(P, P.two_eps_sigma * (q[aa] * n[b] - n[aa] * q[b]), d2, rd2, ld2);
                 f[aa] += w * n[b];
                 f[b] -= w * n[aa];
             }
     }
-    const double mean = div_force(P, f[0] + f[1] + f[2], 3.0, P.r_3);
+    const double mean = div_const(P, f[0] + f[1] + f[2], 3.0, P.r_3, P.l_3);
     const double scale = dt / (local_tau(P, q0, q1, q2) * P.eps);
     Proposal o;
     o.z0 = q0 - scale * (f[0] - mean);
@@ -833,7 +834,7 @@ __device__ __forceinline__ Proposal propose_cell_mixed(const DevParams& P, const
 // bounds.  A cell that equals the reference cell with its neighbours takes the
 // proposal computed at the first such cell of the block.
 template <bool kFindUniform>
-__device__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double& change, bool& mixbad,
+__device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double& change, bool& mixbad,
                               bool& simplexbad) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
@@ -1100,7 +1101,7 @@ __device__ bool phase_mix(const Dom& a, Red& red, int cur, bool& mixbad) {
 // kSolve32: the mixed form's set-up (FP32 copies for the inner solve); the FP64
 // kernel is compiled without it.
 template <bool kSolve32>
-__device__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& rhs2, double& rz, double& rr) {
+__device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& rhs2, double& rz, double& rr) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     double s0 = 0, s1 = 0, s2 = 0;
@@ -1203,7 +1204,7 @@ __device__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& 
 
 // APPLY: p_new = z (first) or z + beta*p_old, written to p[pout]; Ap; <p,Ap>.
 // Slots: wE, wN, z (stencils), chi, p_old (stencil).
-__device__ bool phase_apply(const Dom& a, Red& red, double dt, bool first, double beta, int pout, double& pAp) {
+__device__ __forceinline__ bool phase_apply(const Dom& a, Red& red, double dt, bool first, double beta, int pout, double& pAp) {
     const DevBufs& B = a.B;
     double* pn = B.p[pout];
     double s = 0;
@@ -1270,7 +1271,7 @@ __device__ bool phase_apply(const Dom& a, Red& red, double dt, bool first, doubl
 
 // UPDATE: x += alpha p; r -= alpha Ap; z = r/diag; {<r,z>, <r,r>}.
 // Slots (no stencils): x, p, r, Ap, diag.
-__device__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, double& rz, double& rr) {
+__device__ __forceinline__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, double& rz, double& rr) {
     const DevBufs& B = a.B;
     double s0 = 0, s1 = 0;
     const int maps[5] = {kMapXc, pcur ? kMapP1c : kMapP0c, kMapRc, kMapApc, kMapDiagc};
@@ -1329,7 +1330,7 @@ __device__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, dou
 }
 
 // RESET: z = r/diag; <r,z>  (pearl_serial.cpp:1060-1064)
-__device__ bool phase_reset(const Dom& a, Red& red, double& rz) {
+__device__ __forceinline__ bool phase_reset(const Dom& a, Red& red, double& rz) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     double s = 0;
@@ -1437,7 +1438,7 @@ __device__ __forceinline__ F2 stencil2f(const Src& s, int k, bool v1) {
 // APPLY32: p = z (first) or z + beta p_old into p32[pout]; A p; <p,Ap> in FP64.
 // The FP32 planes are staged through TMA like the FP64 passes' (FP32 boxes,
 // kBoxW32 wide), or read from global memory when staging is off.
-__device__ bool phase_apply32(const Dom& a, Red& red, double dt, bool first, double beta, int pout, double& pAp) {
+__device__ __forceinline__ bool phase_apply32(const Dom& a, Red& red, double dt, bool first, double beta, int pout, double& pAp) {
     const DevBufs& B = a.B;
     float* __restrict__ pn = B.p32[pout];
     float* __restrict__ apo = B.Ap32;
@@ -1504,7 +1505,7 @@ __device__ bool phase_apply32(const Dom& a, Red& red, double dt, bool first, dou
 // (blocks x threads) of the block group, a fixed assignment, so the sums are
 // deterministic; cells of the row padding (x >= nx) keep their values and add
 // nothing.
-__device__ bool phase_update32(const Dom& a, Red& red, double alpha, int pcur, double& rz, double& rr) {
+__device__ __forceinline__ bool phase_update32(const Dom& a, Red& red, double alpha, int pcur, double& rz, double& rr) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     const float* __restrict__ p = B.p32[pcur];
@@ -1556,7 +1557,7 @@ __device__ bool phase_update32(const Dom& a, Red& red, double alpha, int pcur, d
 // RESID32: the FP64 residual r = rhs - A x of the accumulated unknown (as the
 // final update's), handed to the next FP32 round: r32 = r, z32 = r32/diag.
 // Slots: wE, wN, x (stencils), chi, c, icpt.  Reduction {<r,r> FP64, <r32,z32>}.
-__device__ bool phase_resid32(const Dom& a, Red& red, int cur, double dt, double& rr, double& rz) {
+__device__ __forceinline__ bool phase_resid32(const Dom& a, Red& red, int cur, double dt, double& rr, double& rz) {
     const DevBufs& B = a.B;
     double s0 = 0, s1 = 0;
     const int maps[6] = {kMapWE, kMapWN, kMapX, kMapChi, kMapState + 5 * cur + 3, kMapIcpt};
@@ -1588,7 +1589,7 @@ __device__ bool phase_resid32(const Dom& a, Red& red, int cur, double dt, double
 
 // RESET32: after a final update whose true residual missed, that residual
 // (written by FINAL in FP64) starts the next FP32 round.  Reduction {<r32,z32>}.
-__device__ bool phase_reset32(const Dom& a, Red& red, double& rz) {
+__device__ __forceinline__ bool phase_reset32(const Dom& a, Red& red, double& rz) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     double s = 0;
@@ -1617,7 +1618,7 @@ __device__ bool phase_reset32(const Dom& a, Red& red, double& rz) {
 // thread are processed one after the other (this phase carries the most live
 // values).  Slots: wE, wN, x, phi_a, phi_t, phi_g (stencils), c, chi, icpt.
 // Reduction: {closure max, bad max, carbon sum, energy sum, <r,r>}.
-__device__ bool phase_final(const Dom& a, Red& red, int cur, double dt, double& closure, bool& bad,
+__device__ __forceinline__ bool phase_final(const Dom& a, Red& red, int cur, double dt, double& closure, bool& bad,
                             double& mass, double& energy, double& rr) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
@@ -1808,7 +1809,7 @@ constexpr int kMixedMaxRounds = 16;  // FP32 rounds of one mixed solve before th
 // FP64 solve: rr holds the residual estimate of the last pass (FP64 after
 // SETUP, RESID32 and FINAL, FP32 after an inner update); o.it counts FP32
 // iterations.
-__device__ bool diffusion_mixed(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
+__device__ __forceinline__ bool diffusion_mixed(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
     const DevParams& P = a.P;
     double rhs2, rz, rr;
     if (!phase_setup<true>(a, red, cur, dt, rhs2, rz, rr)) return false;
@@ -1864,7 +1865,7 @@ __device__ bool diffusion_mixed(const Dom& a, Red& red, int cur, double dt, Diff
 // kSolve32: the kernel of the mixed solve (diffusion_mixed); the FP64 kernels
 // are compiled without it, so its registers do not weigh on their phases.
 template <bool kSolve32>
-__device__ bool diffusion(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
+__device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
     const DevParams& P = a.P;
     o.ok = false;
     o.it = 0;
@@ -1934,7 +1935,7 @@ struct StepState {
 };
 
 template <bool kSolve32>
-__device__ bool advance(const Dom& a, Red& red, StepState& st, double stop_time, pearl_step_info& info) {
+__device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, double stop_time, pearl_step_info& info) {
     const DevParams& P = a.P;
     double dt = st.S.dt;
     if (P.dt_max < dt) dt = P.dt_max;
@@ -2211,7 +2212,8 @@ __device__ bool phase_smooth_force(const Dom& a, Red& red, int cur, double& forc
                 if ((dir == 2 && y == 0) || (dir == 3 && y == P.ny - 1)) continue;
                 const size_t j = dir == 0 ? iw : (dir == 1 ? ie : (dir == 2 ? is : in));
                 const double n[3] = {ph[0][j], ph[1][j], ph[2][j]};
-                const double d2 = dir < 2 ? P.dx2 : P.dy2, rd2 = dir < 2 ? P.r_dx2 : P.r_dy2;
+                const double d2 = dir < 2 ? P.dx2 : P.dy2;
+        const double rd2 = dir < 2 ? P.r_dx2 : P.r_dy2, ld2 = dir < 2 ? P.l_dx2 : P.l_dy2;
 #pragma unroll
                 for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
@@ -2458,9 +2460,11 @@ __device__ __forceinline__ void init_tiles(Tiles& T, const Dom& a, bool wanted) 
         for (int k = threadIdx.x; k < most; k += kThreads) T.held[k] = 0;
 }
 
-// The persistent step kernel's body; kSolve32 selects the mixed form's inner
-// solve (pearl_kernel_mixed), every other part is the same code.
-template <bool kSolve32>
+// The body of the kernels of one domain.  kRun: the step loop (kSolve32: with
+// the mixed form's inner solve); otherwise every other mode.  The step loop is
+// a kernel of its own because a second copy of the phases in it (the modes that
+// run one of them alone) costs the loop's phases registers.
+template <bool kSolve32, bool kRun>
 __device__ __forceinline__ void step_body(const KArgs& args) {
     const Dom a{args.P, args.B, args.maps, args.use_tma, (int)blockIdx.x, (int)gridDim.x, args.B.ctl, args.B.part,
                 args.shift_trigger, args.shift_target, args.shift_c_gamma, args.smooth_max_steps,
@@ -2475,7 +2479,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     }
     __shared__ Tiles tiles;
     // (a tape takes the whole solution plane of every step)
-    init_tiles(tiles, a, args.mode == kModeRun && !kSolve32 && !args.tape);
+    init_tiles(tiles, a, kRun && !kSolve32 && !args.tape);
     __syncthreads();
     Red red(a, &clk);
     red.pipe_ptr = &pipe;
@@ -2488,7 +2492,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     st.mass0 = ctl->mass0;
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
 
-    if (args.mode == kModeRun) {
+    if constexpr (kRun) {
         long long steps = 0, cg_total = 0;
         int cg_peak = 0, reached = 0;
         pearl_step_info last;
@@ -2529,10 +2533,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
         red.flush();
         return;
     }
-    // the mixed-solve kernel runs only the run mode (the host launches every
-    // other mode, none of which solves, in the FP64 kernel; a second solving
-    // mode here would double the solve's code and its register pressure)
-    if constexpr (kSolve32) return;
+    if constexpr (kRun) return;
     if (args.mode == kModePropose) {
         double change;
         bool mixbad, simplexbad;
@@ -2642,10 +2643,13 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
 }
 
 __global__ void __launch_bounds__(kThreads, kMinBlocks) pearl_kernel(const __grid_constant__ KArgs args) {
-    step_body<false>(args);
+    step_body<false, true>(args);
+}
+__global__ void __launch_bounds__(kThreads, kMinBlocks) pearl_kernel_modes(const __grid_constant__ KArgs args) {
+    step_body<false, false>(args);
 }
 __global__ void __launch_bounds__(kThreads, kMinBlocks) pearl_kernel_mixed(const __grid_constant__ KArgs args) {
-    step_body<true>(args);
+    step_body<true, true>(args);
 }
 
 // ------------------------------------------------------------------ batched instances

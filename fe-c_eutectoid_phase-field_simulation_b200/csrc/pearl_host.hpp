@@ -60,9 +60,11 @@ bool valid_params(const pearl_params* p);
 double host_psi(const pearl_params* p, int a, double mu);
 // Tile of (32 << wx) x (2 warps >> wx) cells: 2^wx warps side by side in x.
 void set_tile_shape(pearl_gpu_ctx* ctx, int wx_log2);
-// The persistent step kernel of a block shape; solve32: the kernel with the
-// mixed form's FP32 inner solve.
-const void* step_kernel(int warps, bool solve32 = false);
+// The kernels of a block shape: the step loop, the step loop with the mixed
+// form's FP32 inner solve, and all other modes; fast_div: DevParams::fast_div of
+// the domain.
+enum StepKernel { kStepRun, kStepRunMixed, kStepModes };
+const void* step_kernel(int warps, StepKernel kind, bool fast_div);
 // Gives the context the kernels of another block shape (tile counts and TMA
 // boxes follow); its own launch grid is kept.
 void set_geometry(pearl_gpu_ctx* ctx, int warps);

@@ -103,6 +103,8 @@ struct AdjArgs {
     __global__ void __launch_bounds__(32 * (WARPS), MIN_BLOCKS)                                                 \
         pearl_kernel_mixed(const __grid_constant__ KArgs args);                                               \
     __global__ void __launch_bounds__(32 * (WARPS), MIN_BLOCKS)                                                 \
+        pearl_kernel_modes(const __grid_constant__ KArgs args);                                               \
+    __global__ void __launch_bounds__(32 * (WARPS), MIN_BLOCKS)                                                 \
         pearl_batch_kernel(const __grid_constant__ BatchArgs args);                                           \
     __global__ void __launch_bounds__(32 * (WARPS), MIN_BLOCKS)                                                 \
         pearl_batch_kernel_mixed(const __grid_constant__ BatchArgs args);                                     \
@@ -115,6 +117,13 @@ namespace g8 {
 PEARL_DECLARE_KERNELS(8, 2)
 }
 namespace g16 {
+PEARL_DECLARE_KERNELS(16, 1)
+}
+// the same with the general division by constants (DevParams::fast_div == 0)
+namespace g8_div {
+PEARL_DECLARE_KERNELS(8, 2)
+}
+namespace g16_div {
 PEARL_DECLARE_KERNELS(16, 1)
 }
 #undef PEARL_DECLARE_KERNELS

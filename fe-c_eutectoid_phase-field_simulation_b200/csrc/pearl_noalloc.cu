@@ -131,9 +131,10 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
     B.part = scratch + kNoAllocPlanes * (size_t)kNoAllocMaxCells;
     B.ctl = reinterpret_cast<Ctl*>(B.part + (size_t)2 * kNoAllocMaxBlocks * kMaxRed);
 
+    const void* const kernel = step_kernel(8, kStepRun, ctx.P.fast_div != 0);
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, g8::pearl_kernel, tile_geometry(8).threads, 0) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tile_geometry(8).threads, 0) !=
             cudaSuccess ||
         per_sm < 1)
         return PEARL_ERR_CUDA;
@@ -158,7 +159,7 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
     a.L.end_time = INFINITY;
     a.L.output_eps = 0;
     void* kargs[] = {&a};
-    if (cudaLaunchCooperativeKernel((const void*)g8::pearl_kernel, dim3(grid), dim3(tile_geometry(8).threads), kargs, 0,
+    if (cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(tile_geometry(8).threads), kargs, 0,
                                     st) !=
         cudaSuccess)
         return PEARL_ERR_CUDA;

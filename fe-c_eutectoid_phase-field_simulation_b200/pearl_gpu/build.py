@@ -26,10 +26,11 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # FP64 path: -fmad=false keeps every multiply and add separately rounded, as in
 # the reference built for plain x86-64, so per-cell results match bitwise.
 # (object, source, flags); the phases and kernels are compiled once per block
-# shape: 8 warps (namespace g8) and 16 warps (namespace g16).
+# shape (8 warps: namespace g8, 16 warps: g16) and per way of dividing by the
+# formulas' constants (two operations, or the general division: g8_div, g16_div).
 CU_SOURCES = [
-    ("pearl_fp64_g8", "pearl_fp64.cu", ["-fmad=false", "-DPEARL_TILE_WARPS=8"]),    # phases and kernels
-    ("pearl_fp64_g16", "pearl_fp64.cu", ["-fmad=false", "-DPEARL_TILE_WARPS=16"]),
+    *((f"pearl_fp64_g{w}" + ("" if fast else "_div"), "pearl_fp64.cu",
+       ["-fmad=false", f"-DPEARL_TILE_WARPS={w}", f"-DPEARL_FAST_DIV={fast}"]) for w in (8, 16) for fast in (1, 0)),
     ("pearl_ctx", "pearl_ctx.cu", ["-fmad=false"]),            # context, transfers, single-domain C ABI
     ("pearl_batch", "pearl_batch.cu", ["-fmad=false"]),        # batched instances
     ("pearl_adjoint_host", "pearl_adjoint_host.cu", ["-fmad=false"]),  # adjoint gradient driver
