@@ -21,8 +21,10 @@ struct Cell {
     bool has[4];     // S and N are absent at the y walls
 };
 
-__device__ __forceinline__ Cell cell_at(const DevParams& P, long long idx) {
-    const int x = (int)(idx % P.nx), y = (int)(idx / P.nx);
+// (32-bit indices: a domain has at most 2e9 cells, and a 64-bit division costs
+// more than most of these passes' arithmetic)
+__device__ __forceinline__ Cell cell_at(const DevParams& P, unsigned idx) {
+    const int y = (int)(idx / (unsigned)P.nx), x = (int)(idx - (unsigned)y * (unsigned)P.nx);
     Cell c;
     const size_t row = (size_t)y * P.pitch;
     c.i = row + x;
@@ -36,9 +38,9 @@ __device__ __forceinline__ Cell cell_at(const DevParams& P, long long idx) {
     return c;
 }
 
-#define FOR_CELLS(P)                                                                                     \
-    for (long long idx_ = (long long)a.bid * kThreads + threadIdx.x; idx_ < (long long)(P).nx * (P).ny; \
-         idx_ += (long long)a.nblk * kThreads)
+#define FOR_CELLS(P)                                                                                        \
+    for (unsigned idx_ = (unsigned)a.bid * kThreads + threadIdx.x; idx_ < (unsigned)(P).nx * (unsigned)(P).ny; \
+         idx_ += (unsigned)a.nblk * kThreads)
 
 // The forces of propose_cell for one cell, with the same arithmetic (so z and
 // the projection's active set equal the forward's bitwise).
@@ -104,7 +106,8 @@ __device__ bool adj_seed(const Dom& a, Red& red, const AdjArgs& g) {
 }
 
 __device__ __forceinline__ double adj_face(const DevParams& P, double k, double kn, int dir) {
-    return 0.5 * (k + kn) / (dir < 2 ? P.dx2 : P.dy2);
+    return dir < 2 ? div_const(P, 0.5 * (k + kn), P.dx2, P.r_dx2, P.l_dx2)
+                   : div_const(P, 0.5 * (k + kn), P.dy2, P.r_dy2, P.l_dy2);
 }
 
 // One reverse step.  s0: state before the step (5 planes); s1: tape slot of the step.
@@ -211,6 +214,7 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
     // P3: diffusion adjoint (c^ = lambda, trial-phi adjoint) fused with the
     // cell-local part of the propose adjoint at the state before the step.
     double gM = 0, gS = 0, gD = 0;
+    const double half_dx2 = 0.5 / P.dx2, half_dy2 = 0.5 / P.dy2;
     FOR_CELLS(P) {
         const Cell c = cell_at(P, idx_);
         const size_t i = c.i;
@@ -220,7 +224,7 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
         for (int d = 0; d < 4; ++d)
             if (c.has[d]) {
                 const size_t j = c.n[d];
-                Kb -= dt * (lam - J.lam[j]) * (ui - u[j]) * (0.5 / (d < 2 ? P.dx2 : P.dy2));
+                Kb -= dt * (lam - J.lam[j]) * (ui - u[j]) * (d < 2 ? half_dx2 : half_dy2);
             }
         const double cb = J.bc[i] - lam;
         double tq[3];
@@ -269,7 +273,7 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
         for (int aa = 0; aa < 3; ++aa) zb[aa] = act[aa] ? gb[aa] - gs / na : 0.0;
         double qb[3] = {zb[0], zb[1], zb[2]};
         const double sbar = -(zb[0] * gg[0] + zb[1] * gg[1] + zb[2] * gg[2]);
-        const double zm = (zb[0] + zb[1] + zb[2]) / 3.0;
+        const double zm = div_const(P, zb[0] + zb[1] + zb[2], 3.0, P.r_3, P.l_3);
         double Fb[3];
 #pragma unroll
         for (int aa = 0; aa < 3; ++aa) Fb[aa] = -sc * (zb[aa] - zm);
@@ -305,13 +309,14 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
         for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
             for (int b = 0; b < 3; ++b)
-                mb += Fb[aa] * dpsim[b] * (dtq[aa] + (b == aa ? 6.0 * q[b] * (1.0 - q[b]) : 0.0)) / P.Vm;
+                mb += div_const(P, Fb[aa] * dpsim[b] * (dtq[aa] + (b == aa ? 6.0 * q[b] * (1.0 - q[b]) : 0.0)), P.Vm,
+                                P.r_Vm, P.l_Vm);
 #pragma unroll
         for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
             for (int cc = 0; cc < 3; ++cc) {
                 const double d = cc != aa ? dsum * 2.0 * q[3 - aa - cc] : dpsi[aa] * (6.0 - 12.0 * q[aa]);
-                qb[cc] += Fb[aa] * d / P.Vm;
+                qb[cc] += div_const(P, Fb[aa] * d, P.Vm, P.r_Vm, P.l_Vm);
             }
         J.bmu[i] = mb;
 #pragma unroll
@@ -327,6 +332,8 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
     grad[2] += v3[2];
     // P4: gradient-term couplings, gathered from the four neighbours
     double gS2 = 0;
+    const double kappa_x = P.two_eps_sigma / P.dx2, kappa_y = P.two_eps_sigma / P.dy2;
+    const double two_eps_x = g.two_eps / P.dx2, two_eps_y = g.two_eps / P.dy2;
     FOR_CELLS(P) {
         const Cell c = cell_at(P, idx_);
         const size_t i = c.i;
@@ -345,8 +352,7 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
             load3p(s0, pe, j, n);
 #pragma unroll
             for (int aa = 0; aa < 3; ++aa) Fj[aa] = J.Fb[aa][j];
-            const double d2 = d < 2 ? P.dx2 : P.dy2;
-            const double kappa = P.two_eps_sigma / d2;
+            const double kappa = d < 2 ? kappa_x : kappa_y;
 #pragma unroll
             for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
@@ -356,7 +362,7 @@ __device__ bool adj_step(const Dom& a, Red& red, const AdjArgs& g, const double*
                     const double Y = Fi[aa] * n[b] - Fi[b] * n[aa];
                     qb[aa] += kappa * n[b] * Y;
                     qb[b] -= kappa * n[aa] * Y;
-                    gS2 += X * Y * (g.two_eps / d2);
+                    gS2 += X * Y * (d < 2 ? two_eps_x : two_eps_y);
                     // the neighbour's forces, in which this cell is the neighbour
                     const double Xj = n[aa] * q[b] - q[aa] * n[b];
                     const double Yj = Fj[aa] * q[b] - Fj[b] * q[aa];
