@@ -20,39 +20,38 @@ namespace pearl_gpu {
 
 namespace division_detail {
 
-inline uint64_t mul_mod(uint64_t a, uint64_t b, uint64_t m) { return (uint64_t)((unsigned __int128)a * b % m); }
-
-// Significands A in [2^52, 2^53) with A 2^s = M B + n, M odd, |n| < 8, where
-// s = 53 for A >= B and 54 for A < B (so that M / 2 is the scaled quotient's
-// midpoint).  Calls f(A) for each until it returns false.
+// Calls f(A) until it returns false for the significands A in [2^52, 2^53) with
+// A 2^s = M B + n, |n| < 8, where s = 53 (for A >= B) or 54 (for A < B): with M
+// odd, M / 2 is a midpoint of the scaled quotient.  (An even M is a quotient
+// next to a double, which f finds right as well: M is not looked at.)
 //
 // The bound on |n|: with zl at most 1.5 units in its last place from 1/b - zh,
 // |zh + zl - 1/b| <= 3 2^-106 / b and the rounding of a*zl adds 2^-106 |a/b|, so
 // the value before the last rounding is within 2^-51 units in the last place of
 // the quotient; a distance of |n| / (2B) >= |n| 2^-54 units below that means
 // |n| < 8.
+//
+// A few hundred nanoseconds: a single step on a small domain pays for nine.
 template <class F>
 bool near_midpoints(uint64_t B, F&& f) {
     int t = 0;
     while (!((B >> t) & 1)) ++t;
+    if (t > 2) return true;  // 2^t divides n
     const uint64_t Bo = B >> t, lo = 1ull << 52, hi = 1ull << 53;
-    if (Bo == 1) return true;  // a power of two divides exactly
-    const uint64_t half = (Bo + 1) / 2;  // 1/2 modulo Bo
+    uint64_t inv64 = Bo;  // 1/Bo modulo 2^64 by Newton's iteration (right to 3 bits at first)
+    for (int k = 0; k < 5; ++k) inv64 *= 2 - Bo * inv64;
     for (int s = 53; s <= 54; ++s) {
-        uint64_t inv = 1;  // 2^-(s - t) modulo Bo
-        for (int k = 0; k < s - t; ++k) inv = mul_mod(inv, half, Bo);
-        for (int n = -7; n <= 7; ++n) {
-            if (n == 0 || n % (1 << (t < 5 ? t : 5)) != 0) continue;  // 2^t has to divide n
-            const int no = n / (1 << (t < 5 ? t : 5));
-            const uint64_t residue = no > 0 ? (uint64_t)no % Bo : (Bo - (uint64_t)(-no) % Bo) % Bo;
-            uint64_t A = mul_mod(residue, inv, Bo);
-            if (A < lo) A += (lo - A + Bo - 1) / Bo * Bo;
-            for (; A < hi; A += Bo) {
-                if ((s == 53) != (A >= B)) continue;
-                const __int128 x = ((__int128)A << s) - n;
-                if (x % B != 0 || !((x / B) & 1)) continue;
-                if (!f(A)) return false;
-            }
+        // 2^-(s - t) modulo Bo: (1 + Bo m) / 2^(s - t) with m = -1/Bo modulo 2^(s - t)
+        const int k = s - t;
+        const uint64_t m = (0 - inv64) & ((1ull << k) - 1);
+        const uint64_t inv = (uint64_t)(((unsigned __int128)Bo * m + 1) >> k);
+        uint64_t r = 0;
+        for (int n = 1; n << t < 8; ++n) {
+            r += inv;
+            if (r >= Bo) r -= Bo;
+            for (uint64_t A : {r, Bo - r})
+                for (A += A < lo ? (lo - A + Bo - 1) / Bo * Bo : 0; A < hi; A += Bo)
+                    if (!f(A)) return false;
         }
     }
     return true;
@@ -63,7 +62,7 @@ bool near_midpoints(uint64_t B, F&& f) {
 // Constants (zh, zl) for the divisor b, true when they give a/b for all normal
 // a with a normal quotient.  zl is 1/b - zh rounded, or a neighbour of it where
 // that one misses a quotient (about one divisor in 160); for one divisor in a
-// thousand none of the three does, and the kernels divide with div_exact.
+// thousand none of the three does, and the kernels of the general division run.
 inline bool exact_reciprocal(double b, double& zh, double& zl) {
     zh = 1.0 / b;
     zl = std::fma(-b, zh, 1.0) / b;  // the residual is exact

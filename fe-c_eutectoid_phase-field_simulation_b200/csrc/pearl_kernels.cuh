@@ -49,6 +49,8 @@ struct KArgs {
     // hist[(hist_next + k) % hist_cap]
     pearl_step_info* hist;
     long long hist_cap, hist_next;
+    // run mode: leave the state in set 0 (the no-allocation step's caller planes)
+    int end_in_set0;
 };
 
 // One instance of a batch: its tensor maps, parameters and buffers.

@@ -158,6 +158,7 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
     a.L.stop_time = stop_time;
     a.L.end_time = INFINITY;
     a.L.output_eps = 0;
+    a.end_in_set0 = 1;  // the accepted state ends in the caller's planes
     void* kargs[] = {&a};
     if (cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(tile_geometry(8).threads), kargs, 0,
                                     st) !=
@@ -168,15 +169,6 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
         return PEARL_ERR_CUDA;
     if (h.status != PEARL_OK) return h.status;
     if (h.steps != 1) return PEARL_ERR_INVALID_ADVANCE_TIME;
-    // The accepted state sits in the scratch set; copy it into the caller's planes.
-    if (h.cur == 1) {
-        if (cudaMemcpyAsync(d_phi, B.phi[1][0], 3 * pe * sizeof(double), cudaMemcpyDeviceToDevice, st) !=
-                cudaSuccess ||
-            cudaMemcpyAsync(d_carbon, B.c[1], pe * sizeof(double), cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-            cudaMemcpyAsync(d_mu, B.mu[1], pe * sizeof(double), cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return PEARL_ERR_CUDA;
-    }
     *scalars = h.S;
     if (out) *out = h.last;
     return PEARL_OK;
