@@ -85,6 +85,10 @@ const void* step_kernel(int warps, StepKernel kind, bool fast_div) {
     return kernels[warps == 16][kind][fast_div];
 }
 
+const void* plain_step_kernel(int grid, int sms) {
+    return grid <= sms ? (const void*)plain_wide::pearl_kernel : (const void*)plain::pearl_kernel;
+}
+
 void set_geometry(pearl_gpu_ctx* ctx, int warps) {
     if (ctx->warps == warps) return;
     ctx->warps = warps;
@@ -213,8 +217,9 @@ int launch(pearl_gpu_ctx* ctx, KArgs& args) {
     if (tma) std::memcpy(args.maps, ctx->maps, sizeof ctx->maps);
     const TileGeometry g = tile_geometry(ctx->warps);
     const StepKernel kind = args.mode != kModeRun ? kStepModes : ctx->P.mixed_cg ? kStepRunMixed : kStepRun;
-    PG_CUDA(ctx, cudaLaunchCooperativeKernel(step_kernel(ctx->warps, kind, ctx->P.fast_div != 0),
-                                             dim3(ctx->grid),
+    const void* kernel = step_kernel(ctx->warps, kind, ctx->P.fast_div != 0);
+    if (kind == kStepRun && !tma && ctx->warps == 8 && ctx->P.fast_div) kernel = plain_step_kernel(ctx->grid, ctx->sms);
+    PG_CUDA(ctx, cudaLaunchCooperativeKernel(kernel, dim3(ctx->grid),
                                              dim3(g.threads), kargs,
                                              tma ? g.tma_smem_bytes : 0, ctx->stream));
     ctx->launches++;
@@ -630,6 +635,7 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     // gets the stage buffers; the grid fits the residency of all
     const void* kernels[6];
     for (int k = 0; k < 6; ++k) kernels[k] = step_kernel(ctx->warps, (StepKernel)(k / 2), k & 1);
+    ctx->sms = sms;
     for (const void* k : kernels)
         if (ctx->use_tma && cudaFuncSetAttribute(k,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -17,14 +17,23 @@
 
 // The device code is compiled for two block shapes (PEARL_TILE_WARPS) and two
 // ways of dividing by the formulas' constants (PEARL_FAST_DIV, see div_const),
-// each in a namespace of its own.
+// each in a namespace of its own.  PEARL_PLAIN adds the step loop of domains that
+// do not stage (8 warps; 2: of those with at most one block per SM), without the
+// staging pipeline's code and registers.
+#ifndef PEARL_PLAIN
+#define PEARL_PLAIN 0
+#endif
 #ifndef PEARL_TILE_WARPS
 #define PEARL_TILE_WARPS 8
 #endif
 #ifndef PEARL_FAST_DIV
 #define PEARL_FAST_DIV 1
 #endif
-#if PEARL_TILE_WARPS == 16
+#if PEARL_PLAIN == 1
+#define PEARL_GEOM_NS plain
+#elif PEARL_PLAIN == 2
+#define PEARL_GEOM_NS plain_wide
+#elif PEARL_TILE_WARPS == 16
 #define PEARL_GEOM_NS PEARL_NS_(g16, PEARL_FAST_DIV)
 #elif PEARL_TILE_WARPS == 8
 #define PEARL_GEOM_NS PEARL_NS_(g8, PEARL_FAST_DIV)
@@ -312,7 +321,12 @@ constexpr size_t kPipeDoubles = kGeom.pipe_doubles;
 // floats per staged FP32 field (128 B aligned)
 constexpr int kFieldStride32 = (int)(((size_t)kBoxW32 * kBoxH * sizeof(float) + 127) / 128 * 128 / sizeof(float));
 constexpr size_t kTmaSmemBytes = kGeom.tma_smem_bytes;
-constexpr int kMinBlocks = kGeom.min_blocks;
+// The wide plain kernel has an SM to a block: 255 registers a thread, enough to
+// work on both cells of a thread at once (kCellUnroll) where the others take one
+// after the other.
+constexpr bool kPlain = PEARL_PLAIN != 0;
+constexpr int kMinBlocks = PEARL_PLAIN == 2 ? 1 : kGeom.min_blocks;
+constexpr int kCellUnroll = PEARL_PLAIN == 2 ? 2 : 1;
 }  // namespace PEARL_GEOM_NS
 
 // Tensor-map slots: state set s fields 0..4 (phi_a, phi_t, phi_g, c, mu) at

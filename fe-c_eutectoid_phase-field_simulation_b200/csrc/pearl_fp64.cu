@@ -351,7 +351,7 @@ struct Red {
     template <int NV>
     __device__ __forceinline__ bool reduce(double (&v)[NV], unsigned ops, int tag) {
         // this thread's plane stores may be read by TMA (async proxy) after the barrier
-        if (a.use_tma) fence_proxy_async();
+        if (!kPlain && a.use_tma) fence_proxy_async();
         double* slot = a.part + (size_t)(counter & 1u) * a.nblk * kMaxRed;
         const bool ok = grid_reduce<NV>(v, ops, slot, a.bid, a.nblk, a.bar, counter);
         ++counter;
@@ -575,7 +575,7 @@ __device__ __forceinline__ bool sweep(const Dom& a, Red& red, const int (&maps)[
     const int G = a.nblk;
     const int nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / G + 1 : 0;
     const auto tile_of = [&](int k) { return a.bid + (reverse ? nb - 1 - k : k) * G; };
-    if (!a.use_tma) {
+    if (kPlain || !a.use_tma) {
         for (int k = 0; k < nb; ++k) {
             const Pair c = pair_of(P, tile_of(k));
             if (!c.v0) continue;
@@ -587,6 +587,7 @@ __device__ __forceinline__ bool sweep(const Dom& a, Red& red, const int (&maps)[
         }
         return true;
     }
+    if constexpr (!kPlain) {
     constexpr size_t kStageElems = kPipeDoubles * sizeof(double) / sizeof(T);
     constexpr int S = (int)(kStageElems / ((size_t)NF * G_::kStride)) < kMaxStages
                           ? (int)(kStageElems / ((size_t)NF * G_::kStride))
@@ -695,6 +696,7 @@ __device__ __forceinline__ bool sweep(const Dom& a, Red& red, const int (&maps)[
             body(src, c);
         }
         tile_end(t);  // every warp is done with stage s: it is refilled next iteration
+    }
     }
     return true;
 }
@@ -917,7 +919,7 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
                 return;
             }
         }
-#pragma unroll 1
+#pragma unroll kCellUnroll
         for (int k = 0; k < 2; ++k) {
             if (k == 1 && !c.v1) break;
             const int y = c.y0 + k;
@@ -1335,7 +1337,7 @@ __device__ __forceinline__ bool phase_reset(const Dom& a, Red& red, double& rz) 
     const DevBufs& B = a.B;
     double s = 0;
     const Tiles& T = *red.tiles;
-    const bool skip = T.active;
+    const bool skip = !kPlain && T.active;
     if (skip) {
         if (threadIdx.x == 0) red.tiles->u.z = T.u.r / T.u.diag;
         __syncthreads();
@@ -1671,7 +1673,7 @@ __device__ __forceinline__ bool phase_final(const Dom& a, Red& red, int cur, dou
             }
         });
     const bool ok = sweep<9>(a, red, maps, planes, 0x3Fu, true, [&](const auto& src, const Pair& c) {
-#pragma unroll 1
+#pragma unroll kCellUnroll
         for (int k = 0; k < 2; ++k) {
             if (k == 1 && !c.v1) break;
             const int y = c.y0 + k;
@@ -1701,7 +1703,7 @@ __device__ __forceinline__ bool phase_final(const Dom& a, Red& red, int cur, dou
     if (!ok) return false;
     double v[5] = {vclos, vbad, vmass, ven, vrr};
     if (!red.reduce<5>(v, OPS5(kMax, kMax, kSum, kSum, kSum), kTagFinal)) return false;
-    if (red.tiles->enabled) {
+    if (!kPlain && red.tiles->enabled) {
         Tiles& T = *red.tiles;
         const int nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
         for (int k = threadIdx.x; k < nb; k += kThreads) {
@@ -1862,9 +1864,185 @@ __device__ __forceinline__ bool diffusion_mixed(const Dom& a, Red& red, int cur,
     return true;
 }
 
+// The implicit diffusion of a domain with at most one tile a block, without
+// staging: the same passes, sums and order as in `diffusion`, with the two
+// cells of a thread kept in registers from SET-UP to the end of the solve.  On
+// such a domain a pass is a round trip to L2 for its operands and a grid
+// reduction.  Here UPDATE has no operand to load, and APPLY only its
+// neighbours' z and old directions.  (Fetching the latter before UPDATE's
+// reduction makes its release wait for them: UPDATE 3.27 -> 3.39 us.)  The
+// planes that neighbours or FINAL read (wE, wN, x, z, p) are written as before.
+// 128x256: APPLY 3.31 -> 2.46 us, UPDATE 3.23 -> 2.36; in a kernel that also
+// stages, its registers cost the other phases what it gains.
+__device__ __forceinline__ bool diffusion_resident(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
+    const DevParams& P = a.P;
+    const DevBufs& B = a.B;
+    const Pair c = pair_of(P, a.bid < P.ntiles ? a.bid : 0);
+    const bool v0 = a.bid < P.ntiles && c.v0, v1 = v0 && c.v1;
+    double x0 = 0, x1 = 0, r0 = 0, r1 = 0, z0 = 0, z1 = 0, p0 = 0, p1 = 0, Ap0 = 0, Ap1 = 0;
+    double chi0 = 0, chi1 = 0, diag0 = 1, diag1 = 1;
+    Faces f0{}, f1{};
+    double v3[3] = {0, 0, 0};
+    if (v0) {
+        GlobalSrc<5> src;
+        src.f[0] = B.K;
+        src.f[1] = B.mu[cur];
+        src.f[2] = B.chi;
+        src.f[3] = B.icpt;
+        src.f[4] = B.c[cur];
+        src.c = c;
+        const S2 K = stencil2(src, 0, c.v1);
+        S2 u = stencil2(src, 1, c.v1);
+        u.c0 -= P.mu_ref; u.c1 -= P.mu_ref; u.w0 -= P.mu_ref; u.e0 -= P.mu_ref;
+        u.w1 -= P.mu_ref; u.e1 -= P.mu_ref; u.s0 -= P.mu_ref; u.n1 -= P.mu_ref;
+        const auto cell = [&](size_t i, double rhs, double Au, double chi, const Faces& f, double u0, double& diag,
+                              double& x, double& r, double& z) {
+            diag = chi + dt * (f.w0 + f.w1 + f.w2 + f.w3);
+            x = u0;
+            r = rhs - Au;
+            z = r / diag;
+            B.wE[i] = f.w1;
+            B.wN[i] = f.w3;
+            B.x[i] = x;
+            B.z[i] = z;
+            v3[0] += rhs * rhs;
+            v3[1] += r * z;
+            v3[2] += r * r;
+        };
+        chi0 = src.v(2, 0, kC);
+        f0 = faces0(P, K, c);
+        cell(c.i0, src.v(4, 0, kC) - src.v(3, 0, kC), apply0(chi0, dt, f0, u), chi0, f0, u.c0, diag0, x0, r0, z0);
+        if (v1) {
+            chi1 = src.v(2, 1, kC);
+            f1 = faces1(P, K, c);
+            cell(c.i1, src.v(4, 1, kC) - src.v(3, 1, kC), apply1(chi1, dt, f1, u), chi1, f1, u.c1, diag1, x1, r1, z1);
+        }
+    }
+    if (!red.reduce<3>(v3, OPS3(kSum, kSum, kSum), kTagSetup)) return false;
+    double rz = v3[1], rr = v3[2];
+    const double tolerance = P.cg_atol + P.cg_rtol * sqrt(v3[0]);
+    bool first = true;
+    double beta = 0;
+    int pbuf = 0;
+    for (int iteration = 0; iteration <= P.cg_max; ++iteration) {
+        o.it = iteration;
+        o.residual = sqrt(rr);
+        if (!isfinite(o.residual)) return true;
+        if (o.residual <= tolerance) {
+            if (!phase_final(a, red, cur, dt, o.closure, o.bad, o.mass, o.energy, rr)) return false;
+            o.residual = sqrt(rr);
+            if (o.residual <= tolerance * 1.05) {
+                o.ok = true;
+                break;
+            }
+            o.closure = 0;
+            o.bad = false;
+            o.mass = 0;
+            o.energy = 0;
+            // RESET from the residual that this thread's FINAL wrote
+            double s = 0;
+            if (v0) {
+                r0 = B.r[c.i0];
+                z0 = r0 / diag0;
+                B.z[c.i0] = z0;
+                s += r0 * z0;
+            }
+            if (v1) {
+                r1 = B.r[c.i1];
+                z1 = r1 / diag1;
+                B.z[c.i1] = z1;
+                s += r1 * z1;
+            }
+            double v[1] = {s};
+            if (!red.reduce<1>(v, kSum, kTagReset)) return false;
+            rz = v[0];
+            first = true;
+            continue;
+        }
+        if (iteration == P.cg_max) break;
+        const double* const po = B.p[pbuf];
+        pbuf ^= 1;
+        double* const pn = B.p[pbuf];
+        double v[1] = {0};
+        if (v0) {
+            S2 p, q{};
+            if (!first) {
+                q.w0 = po[c.iw0];
+                q.e0 = po[c.ie0];
+                q.s0 = po[c.is0];
+                if (v1) {
+                    q.w1 = po[c.iw1];
+                    q.e1 = po[c.ie1];
+                    q.n1 = po[c.in1];
+                }
+            }
+            p.c0 = z0;
+            p.w0 = B.z[c.iw0];
+            p.e0 = B.z[c.ie0];
+            p.s0 = B.z[c.is0];
+            p.c1 = v1 ? z1 : z0;
+            p.w1 = v1 ? B.z[c.iw1] : 0;
+            p.e1 = v1 ? B.z[c.ie1] : 0;
+            p.n1 = v1 ? B.z[c.in1] : 0;
+            if (!first) {
+                p.c0 = p.c0 + beta * p0;
+                p.c1 = p.c1 + beta * (v1 ? p1 : p0);
+                p.w0 = p.w0 + beta * q.w0;
+                p.e0 = p.e0 + beta * q.e0;
+                p.w1 = p.w1 + beta * q.w1;
+                p.e1 = p.e1 + beta * q.e1;
+                p.s0 = p.s0 + beta * q.s0;
+                p.n1 = p.n1 + beta * q.n1;
+            }
+            p0 = p.c0;
+            Ap0 = apply0(chi0, dt, f0, p);
+            pn[c.i0] = p0;
+            v[0] += p0 * Ap0;
+            if (v1) {
+                p1 = p.c1;
+                Ap1 = apply1(chi1, dt, f1, p);
+                pn[c.i1] = p1;
+                v[0] += p1 * Ap1;
+            }
+        }
+        if (!red.reduce<1>(v, kSum, kTagApply)) return false;
+        const double pAp = v[0];
+        if (!(pAp > 0) || !isfinite(pAp) || !isfinite(rz)) return true;
+        const double alpha = rz / pAp;
+        double v2[2] = {0, 0};
+        if (v0) {
+            x0 = x0 + alpha * p0;
+            r0 = r0 - alpha * Ap0;
+            z0 = r0 / diag0;
+            B.x[c.i0] = x0;
+            B.z[c.i0] = z0;
+            v2[0] += r0 * z0;
+            v2[1] += r0 * r0;
+        }
+        if (v1) {
+            x1 = x1 + alpha * p1;
+            r1 = r1 - alpha * Ap1;
+            z1 = r1 / diag1;
+            B.x[c.i1] = x1;
+            B.z[c.i1] = z1;
+            v2[0] += r1 * z1;
+            v2[1] += r1 * r1;
+        }
+        if (!red.reduce<2>(v2, OPS2(kSum, kSum), kTagUpdate)) return false;
+        rr = v2[1];
+        beta = v2[0] / rz;
+        rz = v2[0];
+        first = false;
+    }
+    if (!o.ok) return true;
+    o.ok = o.closure <= P.closure_tol;
+    return true;
+}
+
 // kSolve32: the kernel of the mixed solve (diffusion_mixed); the FP64 kernels
 // are compiled without it, so its registers do not weigh on their phases.
-template <bool kSolve32>
+// kResident: with diffusion_resident (the step loop of one domain has it).
+template <bool kSolve32, bool kResident>
 __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
     const DevParams& P = a.P;
     o.ok = false;
@@ -1876,6 +2054,9 @@ __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, doubl
     o.energy = 0;
     if constexpr (kSolve32) {
         return diffusion_mixed(a, red, cur, dt, o);
+    }
+    if constexpr (kResident) {
+        if (P.ntiles <= a.nblk) return diffusion_resident(a, red, cur, dt, o);
     }
     double rhs2, rz, rr;
     if (!phase_setup<false>(a, red, cur, dt, rhs2, rz, rr)) return false;
@@ -1906,7 +2087,7 @@ __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, doubl
         if (iteration == P.cg_max) break;
         // the direction of iteration i has spread i + 1 cells into the rim; past the
         // rim, uniform tiles are no longer uniform
-        if (red.tiles->active && iteration + 1 >= kReach && !phase_expand(a, red, pbuf)) return false;
+        if (!kPlain && red.tiles->active && iteration + 1 >= kReach && !phase_expand(a, red, pbuf)) return false;
         const int pout = pbuf ^ 1;
         double pAp;
         if (!phase_apply(a, red, dt, first, beta, pout, pAp)) return false;
@@ -1934,7 +2115,7 @@ struct StepState {
     double e0, mass0;
 };
 
-template <bool kSolve32>
+template <bool kSolve32, bool kResident>
 __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, double stop_time, pearl_step_info& info) {
     const DevParams& P = a.P;
     double dt = st.S.dt;
@@ -1963,7 +2144,7 @@ __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, d
         out.retries = attempt;
         out.accepted_dt = dt;
         bool mixbad, simplexbad;
-        if (!phase_propose<!kSolve32>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
+        if (!phase_propose<!kSolve32 && !kPlain>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
         if (simplexbad) {
             set_error(a, PEARL_ERR_SIMPLEX, 0);
             return false;
@@ -1981,8 +2162,8 @@ __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, d
                 if (!phase_final_phase_only(a, red, st.cur, bad, e1)) return false;
             } else {
                 DiffusionOut d;
-                if (!kSolve32 && red.tiles->enabled) classify_tiles(a, *red.tiles);
-                if (!diffusion<kSolve32>(a, red, st.cur, dt, d)) return false;
+                if (!kSolve32 && !kPlain && red.tiles->enabled) classify_tiles(a, *red.tiles);
+                if (!diffusion<kSolve32, kResident>(a, red, st.cur, dt, d)) return false;
                 good = d.ok;
                 out.cg_iterations = d.it;
                 out.linear_residual = d.residual;
@@ -2015,7 +2196,7 @@ __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, d
             st.S.dt = grown < P.dt_max ? grown : P.dt_max;
             st.cur ^= 1;
             // after more iterations than this what is not uniform may have moved by a tile
-            if (red.tiles->known && out.cg_iterations + 1 >= kReach) {
+            if (!kPlain && red.tiles->known && out.cg_iterations + 1 >= kReach) {
                 __syncthreads();
                 if (threadIdx.x == 0) red.tiles->known = 0;
                 __syncthreads();
@@ -2490,7 +2671,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     __shared__ PhaseClock clk;
     extern __shared__ __align__(128) unsigned char dsmem[];
     Pipe pipe = make_pipe(dsmem);
-    if (a.use_tma) {
+    if (!kPlain && a.use_tma) {
         if (threadIdx.x == 0) init_pipe(pipe);
         __syncthreads();
     }
@@ -2522,7 +2703,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
             }
             pearl_step_info info;
             if (args.forced_dt) st.S.dt = args.forced_dt[steps];
-            if (!advance<kSolve32>(a, red, st, args.L.stop_time, info)) break;
+            if (!advance<kSolve32, kPlain>(a, red, st, args.L.stop_time, info)) break;
             if (args.dt_log && leader) args.dt_log[steps] = info.accepted_dt;
             if (args.hist && leader) args.hist[(args.hist_next + steps) % args.hist_cap] = info;
             if (args.tape) record_tape(a, st.cur, args.tape + args.tape_slot * steps);
@@ -2558,7 +2739,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     if (args.mode == kModePropose) {
         double change;
         bool mixbad, simplexbad;
-        if (!phase_propose<!kSolve32>(a, red, st.cur, args.dt, change, mixbad, simplexbad)) return;
+        if (!phase_propose<!kSolve32 && !kPlain>(a, red, st.cur, args.dt, change, mixbad, simplexbad)) return;
         if (leader) {
             ctl->out[0] = change;
             ctl->iout[0] = mixbad;
@@ -2576,7 +2757,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     }
     if (args.mode == kModeDiffusion) {
         DiffusionOut d;
-        if (!diffusion<kSolve32>(a, red, st.cur, args.dt, d)) return;
+        if (!diffusion<kSolve32, false>(a, red, st.cur, args.dt, d)) return;
         if (leader) {
             ctl->iout[0] = d.ok;
             ctl->iout[1] = d.it;
@@ -2666,6 +2847,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
 __global__ void __launch_bounds__(kThreads, kMinBlocks) pearl_kernel(const __grid_constant__ KArgs args) {
     step_body<false, true>(args);
 }
+#if !PEARL_PLAIN
 __global__ void __launch_bounds__(kThreads, kMinBlocks) pearl_kernel_modes(const __grid_constant__ KArgs args) {
     step_body<false, false>(args);
 }
@@ -2732,7 +2914,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
                 break;
             }
             pearl_step_info info;
-            if (!advance<kSolve32>(a, red, st, args.L.stop_time, info)) {
+            if (!advance<kSolve32, false>(a, red, st, args.L.stop_time, info)) {
                 failed = true;
                 break;
             }
@@ -2803,6 +2985,7 @@ __global__ void wait_limit_selftest_kernel(Ctl* ctl) {
 }
 
 #include "pearl_adjoint.cuh"
+#endif  // !PEARL_PLAIN
 
 }  // namespace PEARL_GEOM_NS
 }  // namespace pearl_gpu

@@ -37,6 +37,7 @@ struct pearl_gpu_ctx {
     double* d_stage = nullptr;  // dense device staging of one host state (5 n doubles)
     size_t stage_elems = 0;
     int grid = 0;
+    int sms = 0;  // of the device
     long long launches = 0;
     double last_ms = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -65,6 +66,9 @@ void set_tile_shape(pearl_gpu_ctx* ctx, int wx_log2);
 // the domain.
 enum StepKernel { kStepRun, kStepRunMixed, kStepModes };
 const void* step_kernel(int warps, StepKernel kind, bool fast_div);
+// The step loop of a domain of 8-warp blocks that does not stage: compiled for
+// one block per SM where the grid allows that, else for two.
+const void* plain_step_kernel(int grid, int sms);
 // Gives the context the kernels of another block shape (tile counts and TMA
 // boxes follow); its own launch grid is kept.
 void set_geometry(pearl_gpu_ctx* ctx, int warps);

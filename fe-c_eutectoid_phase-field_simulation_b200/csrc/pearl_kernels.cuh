@@ -128,6 +128,13 @@ PEARL_DECLARE_KERNELS(8, 2)
 namespace g16_div {
 PEARL_DECLARE_KERNELS(16, 1)
 }
+// The step loop of one domain that does not stage: two blocks per SM, and one.
+namespace plain {
+__global__ void __launch_bounds__(256, 2) pearl_kernel(const __grid_constant__ KArgs args);
+}
+namespace plain_wide {
+__global__ void __launch_bounds__(256, 1) pearl_kernel(const __grid_constant__ KArgs args);
+}
 #undef PEARL_DECLARE_KERNELS
 static_assert(tile_geometry(8).min_blocks == 2 && tile_geometry(16).min_blocks == 1, "kernel launch bounds");
 

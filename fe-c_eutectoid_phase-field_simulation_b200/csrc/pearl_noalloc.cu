@@ -131,10 +131,11 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
     B.part = scratch + kNoAllocPlanes * (size_t)kNoAllocMaxCells;
     B.ctl = reinterpret_cast<Ctl*>(B.part + (size_t)2 * kNoAllocMaxBlocks * kMaxRed);
 
-    const void* const kernel = step_kernel(8, kStepRun, ctx.P.fast_div != 0);
     int sms = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tile_geometry(8).threads, 0) !=
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return PEARL_ERR_CUDA;
+    const void* const kernel =
+        ctx.P.fast_div ? plain_step_kernel(ctx.P.ntiles, sms) : step_kernel(8, kStepRun, false);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tile_geometry(8).threads, 0) !=
             cudaSuccess ||
         per_sm < 1)
         return PEARL_ERR_CUDA;
