@@ -617,13 +617,19 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (!coop) return bail(PEARL_ERR_NO_DEVICE);
-    // Block shape: 16 warps (512 threads, one block per SM, 32x32 tiles) when the
-    // domain gives every SM at least four such tiles, 8 warps (two 256-thread
-    // blocks per SM, 32x16 tiles) for smaller domains, which need the finer
-    // split; PEARL_GPU_TILE_WARPS = 8 or 16 overrides.
+    // Block shape: 8 warps (two 256-thread blocks per SM, 32x16 tiles) up to 160
+    // 32x32 tiles per SM, 16 warps (512 threads, one block per SM, 32x32 tiles)
+    // beyond.  With uniform tiles left out, the finer tiles follow the dense part
+    // of a domain more closely (ms per step, 8 against 16 warps, front at 0.1 and
+    // 0.5 of the height: 1000x1537, 10 tiles per SM, 0.152 against 0.169, at 0.45
+    // 0.250 against 0.266; 2048x4096, 55 tiles, at its start 0.195 against 0.231,
+    // 0.872 against 0.888; 4096x4096, 111 tiles, 0.506 against 0.565, 1.690 against
+    // 1.696); on the largest domains half the blocks in every barrier and 5% fewer
+    // halo bytes count more (4096x8192, 221 tiles, 0.848 against 0.889 at 0.1 but
+    // 3.315 against 3.216 at 0.5).  PEARL_GPU_TILE_WARPS = 8 or 16 overrides.
     {
         const long long tiles16 = (long long)((nx + 31) / 32) * ((ny + 31) / 32);
-        ctx->warps = tiles16 >= 4LL * sms ? 16 : 8;
+        ctx->warps = tiles16 >= 160LL * sms ? 16 : 8;
         if (const char* e = std::getenv("PEARL_GPU_TILE_WARPS")) ctx->warps = std::atoi(e) == 16 ? 16 : 8;
     }
     fill_dev_params(ctx);

@@ -2394,7 +2394,7 @@ __device__ bool phase_smooth_force(const Dom& a, Red& red, int cur, double& forc
                 const size_t j = dir == 0 ? iw : (dir == 1 ? ie : (dir == 2 ? is : in));
                 const double n[3] = {ph[0][j], ph[1][j], ph[2][j]};
                 const double d2 = dir < 2 ? P.dx2 : P.dy2;
-        const double rd2 = dir < 2 ? P.r_dx2 : P.r_dy2, ld2 = dir < 2 ? P.l_dx2 : P.l_dy2;
+        const double rd2 = dir < 2 ? P.r_dx2 : P.r_dy2;
 #pragma unroll
                 for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
