@@ -670,11 +670,11 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     // state: 2 x (3 phi + c + mu); work: K chi icpt diag x r z p0 p1 Ap  -> 20 planes
     const size_t pe = plane_elems(ctx);
     const int nplanes = 22;
-    // reduction partials, then the tiles' marks (one byte each, for the finer of the two tile shapes)
+    // reduction partials, then the tiles' marks and classes (a byte each, for the finer of the two tile shapes)
     const size_t part = (size_t)2 * ctx->grid * kMaxRed;
     const size_t marks = ((size_t)((nx + 31) / 32) * ((ny + 15) / 16) + 7) / 8;
-    if (cudaMalloc(&ctx->slab, (nplanes * pe + part + marks) * sizeof(double)) != cudaSuccess) return bail(PEARL_ERR_CUDA);
-    if (cudaMemset(ctx->slab, 0, (nplanes * pe + part + marks) * sizeof(double)) != cudaSuccess) return bail(PEARL_ERR_CUDA);
+    if (cudaMalloc(&ctx->slab, (nplanes * pe + part + 2 * marks) * sizeof(double)) != cudaSuccess) return bail(PEARL_ERR_CUDA);
+    if (cudaMemset(ctx->slab, 0, (nplanes * pe + part + 2 * marks) * sizeof(double)) != cudaSuccess) return bail(PEARL_ERR_CUDA);
     double* q = ctx->slab;
     for (int s = 0; s < 2; ++s) {
         for (int a = 0; a < 3; ++a, q += pe) ctx->B.phi[s][a] = q;
@@ -697,6 +697,7 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     ctx->B.wN = q; q += pe;
     ctx->B.part = q;
     ctx->B.mixed_tile = reinterpret_cast<unsigned char*>(q + part);
+    ctx->B.tile_class = ctx->B.mixed_tile + marks * sizeof(double);
     if (cudaMalloc(&ctx->d_ctl, sizeof(Ctl)) != cudaSuccess) return bail(PEARL_ERR_CUDA);
     if (cudaMallocHost(&ctx->h_ctl, sizeof(Ctl)) != cudaSuccess) return bail(PEARL_ERR_CUDA);
     std::memset(ctx->h_ctl, 0, sizeof(Ctl));

@@ -158,6 +158,7 @@ struct DevBufs {
     double* wN;    // north-face weight .5*(K+K_north)/dy^2, zero at the top wall
     double* part;  // [2][grid][kMaxRed] block partials
     unsigned char* mixed_tile;  // [ntiles] 1 where a tile is not uniform (Tiles); null: every tile is dense
+    unsigned char* tile_class;  // [ntiles] TileClass of the current attempt (mixed solve)
     struct Ctl* ctl;
     // FP32 planes of the mixed-precision solve (null until a context is put in a
     // mixed-solve precision): the solve's face weights, susceptibility and

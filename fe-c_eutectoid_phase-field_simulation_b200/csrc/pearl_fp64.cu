@@ -291,6 +291,8 @@ struct Uniform {
     Faces f;
     double x, r, z, p, Ap, diag, cn, mun, closure;
     bool held;  // the trial set already holds (mun, cn) in every uniform tile
+    // the mixed solve's FP32 values
+    float wE32, wN32, chi32, diag32, r32, z32, p32, Ap32;
     double add[3];  // the cell's contributions to the current pass's sums
     int bad;
 };
@@ -1022,6 +1024,8 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
 // PROPOSE left (all blocks', after its reduction).  A tile within one tile of a
 // marked one is dense, within two a border tile, four or more away far; a last column narrower than
 // the rim counts with the column beyond it (x is periodic).
+// kMap: also into the domain's map, for a pass that does not walk its own tiles.
+template <bool kMap>
 __device__ void classify_tiles(const Dom& a, Tiles& T) {
     const DevParams& P = a.P;
     const int nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
@@ -1048,10 +1052,13 @@ __device__ void classify_tiles(const Dom& a, Tiles& T) {
         __syncwarp();
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) nearest = min(nearest, __shfl_xor_sync(0xffffffffu, nearest, o));
-        if (k < nb && dy == -3)
-            T.cls[k] = (unsigned char)((nearest <= 1 ? kDense : nearest == 2 ? kBorder : kUniform) |
-                                       (nearest >= 4 ? kFar : 0) |
-                                       (rest < kTileX && bx == P.ntx - 1 ? kLastColumn : 0));
+        if (k < nb && dy == -3) {
+            const unsigned char c = (unsigned char)((nearest <= 1 ? kDense : nearest == 2 ? kBorder : kUniform) |
+                                                    (nearest >= 4 ? kFar : 0) |
+                                                    (rest < kTileX && bx == P.ntx - 1 ? kLastColumn : 0));
+            T.cls[k] = c;
+            if (kMap) a.B.tile_class[a.bid + k * a.nblk] = c;
+        }
     }
     __syncthreads();
     list_tiles(T, nb, [&](int k) { return (T.cls[k] & kClassMask) == kDense; });
@@ -1110,7 +1117,7 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
     const int maps[5] = {kMapK, kMapState + 5 * cur + 4, kMapChi, kMapIcpt, kMapState + 5 * cur + 3};
     const double* const planes[5] = {B.K, B.mu[cur], B.chi, B.icpt, B.c[cur]};
     Uniform& U = red.tiles->u;
-    const auto uni = uniform_pass<!kSolve32>(
+    const auto uni = uniform_pass<true>(
         [&] {
             U.x = U.ref[3] - P.mu_ref;
             const double wx = face_x(P, U.K, U.K), wy = face_y(P, U.K, U.K);
@@ -1119,10 +1126,20 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
             U.diag = U.chi + dt * (U.f.w0 + U.f.w1 + U.f.w2 + U.f.w3);
             const double rhs = U.ref[4] - U.icpt;
             U.r = rhs - Au;
-            U.z = U.r / U.diag;
             U.add[0] = rhs * rhs;
-            U.add[1] = U.r * U.z;
             U.add[2] = U.r * U.r;
+            if constexpr (kSolve32) {
+                U.wE32 = (float)U.f.w1;
+                U.wN32 = (float)U.f.w3;
+                U.chi32 = (float)U.chi;
+                U.diag32 = (float)U.diag;
+                U.r32 = (float)U.r;
+                U.z32 = __fdiv_rn(U.r32, U.diag32);
+                U.add[1] = (double)U.r32 * (double)U.z32;
+            } else {
+                U.z = U.r / U.diag;
+                U.add[1] = U.r * U.z;
+            }
         },
         [&](int n) {
             add_run<3>(n, U.add, s0, s1, s2);
@@ -1144,7 +1161,13 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
                 B.wE[i] = U.f.w1;
                 B.wN[i] = U.f.w3;
                 B.x[i] = U.x;
-                B.z[i] = U.z;
+                if constexpr (kSolve32) {
+                    B.wE32[i] = U.wE32;
+                    B.wN32[i] = U.wN32;
+                    B.z32[i] = U.z32;
+                } else {
+                    B.z[i] = U.z;
+                }
             }
         });
     const bool ok = sweep<5>(a, red, maps, planes, 0x3u, false, [&](const auto& src, const Pair& c) {
@@ -1364,6 +1387,7 @@ __device__ __forceinline__ bool phase_reset(const Dom& a, Red& red, double& rz) 
 
 // EXPAND: a solve whose search direction has spread through the rim writes the
 // planes of its uniform and border tiles and goes on dense (see Tiles).
+template <bool kSolve32>
 __device__ bool phase_expand(const Dom& a, Red& red, int pcur) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
@@ -1379,11 +1403,21 @@ __device__ bool phase_expand(const Dom& a, Red& red, int pcur) {
             B.icpt[i] = U.icpt;
             B.wE[i] = U.f.w1;
             B.wN[i] = U.f.w3;
-            B.diag[i] = U.diag;
             B.x[i] = U.x;
-            B.r[i] = U.r;
-            B.z[i] = U.z;
-            B.p[pcur][i] = U.p;
+            if constexpr (kSolve32) {
+                B.wE32[i] = U.wE32;
+                B.wN32[i] = U.wN32;
+                B.chi32[i] = U.chi32;
+                B.diag32[i] = U.diag32;
+                B.r32[i] = U.r32;
+                B.z32[i] = U.z32;
+                B.p32[pcur][i] = U.p32;
+            } else {
+                B.diag[i] = U.diag;
+                B.r[i] = U.r;
+                B.z[i] = U.z;
+                B.p[pcur][i] = U.p;
+            }
         }
     }
     double v[1] = {0};
@@ -1480,17 +1514,37 @@ __device__ __forceinline__ bool phase_apply32(const Dom& a, Red& red, double dt,
             s += (double)p.c1 * (double)ap1;
         }
     };
+    Uniform& U = red.tiles->u;
+    const auto uni = uniform_pass<true>(
+        [&] {
+            U.p32 = first ? U.z32 : __fmaf_rn(bf, U.p32, U.z32);
+            U.Ap32 = apply32_at(U.chi32, dtf, U.wE32, U.wE32, U.wN32, U.wN32, U.p32, U.p32, U.p32, U.p32, U.p32);
+            U.add[0] = (double)U.p32 * (double)U.Ap32;
+        },
+        [&](int n) {
+            add_run<1>(n, U.add, s, s, s);
+            return true;
+        },
+        [&](int, int t, int cls, bool valid) {
+            if (!valid) return;
+            s += U.add[0];
+            s += U.add[0];
+            if (cls != kBorder) return;
+            const Pair c = pair_of(a.P, t);
+            pn[c.i0] = U.p32;
+            pn[c.i1] = U.p32;
+        });
     // a first iteration stages no old direction (a single five-field sweep for
     // both cases has fewer spills but measured 1 % slower on the mixed step)
     bool ok;
     if (first) {
         const int maps[4] = {kMap32WE, kMap32WN, kMap32Z, kMap32Chi};
         const float* const planes[4] = {B.wE32, B.wN32, B.z32, B.chi32};
-        ok = sweep<4, false, float>(a, red, maps, planes, 0x7u, true, body);
+        ok = sweep<4, false, float>(a, red, maps, planes, 0x7u, true, body, uni);
     } else {
         const int maps[5] = {kMap32WE, kMap32WN, kMap32Z, kMap32Chi, pout ? kMap32P0 : kMap32P1};
         const float* const planes[5] = {B.wE32, B.wN32, B.z32, B.chi32, B.p32[pout ^ 1]};
-        ok = sweep<5, false, float>(a, red, maps, planes, 0x17u, true, body);
+        ok = sweep<5, false, float>(a, red, maps, planes, 0x17u, true, body, uni);
     }
     if (!ok) return false;
     double v[1] = {s};
@@ -1506,7 +1560,8 @@ __device__ __forceinline__ bool phase_apply32(const Dom& a, Red& red, double dt,
 // in flight without a staging pipeline.  Group g belongs to thread g mod
 // (blocks x threads) of the block group, a fixed assignment, so the sums are
 // deterministic; cells of the row padding (x >= nx) keep their values and add
-// nothing.
+// nothing.  A group lies in one tile, whose class comes from the domain's map:
+// the groups of uniform tiles only add their value.
 __device__ __forceinline__ bool phase_update32(const Dom& a, Red& red, double alpha, int pcur, double& rz, double& rr) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
@@ -1518,12 +1573,36 @@ __device__ __forceinline__ bool phase_update32(const Dom& a, Red& red, double al
     double* __restrict__ x = B.x;
     const float af = (float)alpha;
     double s0 = 0, s1 = 0;
-    const int gpr = P.pitch / 4;
-    const long long ng = (long long)gpr * P.ny;
-    for (long long g = (long long)a.bid * kThreads + threadIdx.x; g < ng; g += (long long)a.nblk * kThreads) {
-        const int y = (int)(g / gpr), x0 = (int)(g % gpr) * 4;
+    Uniform& U = red.tiles->u;
+    const bool skip = red.tiles->active;
+    if (skip) {
+        if (threadIdx.x == 32) {
+            U.x = U.x + alpha * (double)U.p32;
+            U.r32 = __fmaf_rn(-af, U.Ap32, U.r32);
+            U.z32 = __fdiv_rn(U.r32, U.diag32);
+            U.add[0] = (double)U.r32 * (double)U.z32;
+            U.add[1] = (double)U.r32 * (double)U.r32;
+        }
+        __syncthreads();
+    }
+    const unsigned gpr = (unsigned)P.pitch / 4;
+    const unsigned ng = gpr * (unsigned)P.ny;  // fewer than 2^29: a domain has at most 2e9 cells
+    for (unsigned g = (unsigned)a.bid * kThreads + threadIdx.x; g < ng; g += (unsigned)a.nblk * kThreads) {
+        const int y = (int)(g / gpr), x0 = (int)(g - (unsigned)y * gpr) * 4;
         if (x0 >= P.nx) continue;
         const size_t i = (size_t)y * P.pitch + x0;
+        const int cls = skip ? B.tile_class[(size_t)(y >> kTileRowsLog2) * P.ntx + (x0 >> 5)] & kClassMask : kDense;
+        if (cls != kDense) {
+            for (int c = 0; c < 4 && x0 + c < P.nx; ++c) {
+                s0 += U.add[0];
+                s1 += U.add[1];
+                if (cls == kBorder) {
+                    x[i + c] = U.x;
+                    z32[i + c] = U.z32;
+                }
+            }
+            continue;
+        }
         const float4 pv = *reinterpret_cast<const float4*>(p + i);
         const float4 av = *reinterpret_cast<const float4*>(ap + i);
         const float4 dv = *reinterpret_cast<const float4*>(dg + i);
@@ -1564,6 +1643,30 @@ __device__ __forceinline__ bool phase_resid32(const Dom& a, Red& red, int cur, d
     double s0 = 0, s1 = 0;
     const int maps[6] = {kMapWE, kMapWN, kMapX, kMapChi, kMapState + 5 * cur + 3, kMapIcpt};
     const double* const planes[6] = {B.wE, B.wN, B.x, B.chi, B.c[cur], B.icpt};
+    Uniform& U = red.tiles->u;
+    const auto uni = uniform_pass<true>(
+        [&] {
+            U.r = (U.ref[4] - U.icpt) - apply_at(U.chi, dt, U.f, U.x, U.x, U.x, U.x, U.x);
+            U.r32 = (float)U.r;
+            U.z32 = __fdiv_rn(U.r32, U.diag32);
+            U.add[0] = U.r * U.r;
+            U.add[1] = (double)U.r32 * (double)U.z32;
+        },
+        [&](int n) {
+            add_run<2>(n, U.add, s0, s1, s1);
+            return true;
+        },
+        [&](int, int t, int cls, bool valid) {
+            if (!valid) return;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                s0 += U.add[0];
+                s1 += U.add[1];
+            }
+            if (cls != kBorder) return;
+            const Pair c = pair_of(a.P, t);
+            B.z32[c.i0] = B.z32[c.i1] = U.z32;
+        });
     const bool ok = sweep<6>(a, red, maps, planes, 0x7u, true, [&](const auto& src, const Pair& c) {
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {
@@ -1580,7 +1683,7 @@ __device__ __forceinline__ bool phase_resid32(const Dom& a, Red& red, int cur, d
             s0 += r * r;
             s1 += (double)r32 * (double)z32;
         }
-    });
+    }, uni);
     if (!ok) return false;
     double v[2] = {s0, s1};
     if (!red.reduce<2>(v, OPS2(kSum, kSum), kTagTrueRes)) return false;
@@ -1595,14 +1698,28 @@ __device__ __forceinline__ bool phase_reset32(const Dom& a, Red& red, double& rz
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     double s = 0;
+    const Tiles& T = *red.tiles;
+    const bool skip = T.active;
+    if (skip) {
+        if (threadIdx.x == 0) {
+            Uniform& U = red.tiles->u;
+            U.r32 = (float)U.r;
+            U.z32 = __fdiv_rn(U.r32, U.diag32);
+        }
+        __syncthreads();
+    }
+    int pos = 0;
     FOR_TILES(P) {
         const Pair c = pair_of(P, t);
+        const int cls = skip ? T.cls[pos] & kClassMask : kDense;
+        ++pos;
         for (int k = 0; k < 2; ++k) {
             if (!(k ? c.v1 : c.v0)) continue;
             const size_t i = k ? c.i1 : c.i0;
-            const float r32 = (float)B.r[i], z32 = __fdiv_rn(r32, B.diag32[i]);
-            B.r32[i] = r32;
-            B.z32[i] = z32;
+            const float r32 = cls == kDense ? (float)B.r[i] : T.u.r32;
+            const float z32 = cls == kDense ? __fdiv_rn(r32, B.diag32[i]) : T.u.z32;
+            if (cls == kDense) B.r32[i] = r32;
+            if (cls != kUniform) B.z32[i] = z32;
             s += (double)r32 * (double)z32;
         }
     }
@@ -1842,6 +1959,7 @@ __device__ __forceinline__ bool diffusion_mixed(const Dom& a, Red& red, int cur,
             if (!phase_resid32(a, red, cur, dt, rr, rz)) return false;
         } else {
             if (it >= P.cg_max) return true;
+            if (red.tiles->active && it + 1 >= kReach && !phase_expand<true>(a, red, pbuf)) return false;
             const int pout = pbuf ^ 1;
             double pAp;
             if (!phase_apply32(a, red, dt, first, beta, pout, pAp)) return false;
@@ -2087,7 +2205,7 @@ __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, doubl
         if (iteration == P.cg_max) break;
         // the direction of iteration i has spread i + 1 cells into the rim; past the
         // rim, uniform tiles are no longer uniform
-        if (!kPlain && red.tiles->active && iteration + 1 >= kReach && !phase_expand(a, red, pbuf)) return false;
+        if (!kPlain && red.tiles->active && iteration + 1 >= kReach && !phase_expand<false>(a, red, pbuf)) return false;
         const int pout = pbuf ^ 1;
         double pAp;
         if (!phase_apply(a, red, dt, first, beta, pout, pAp)) return false;
@@ -2144,7 +2262,7 @@ __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, d
         out.retries = attempt;
         out.accepted_dt = dt;
         bool mixbad, simplexbad;
-        if (!phase_propose<!kSolve32 && !kPlain>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
+        if (!phase_propose<!kPlain>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
         if (simplexbad) {
             set_error(a, PEARL_ERR_SIMPLEX, 0);
             return false;
@@ -2162,7 +2280,7 @@ __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, d
                 if (!phase_final_phase_only(a, red, st.cur, bad, e1)) return false;
             } else {
                 DiffusionOut d;
-                if (!kSolve32 && !kPlain && red.tiles->enabled) classify_tiles(a, *red.tiles);
+                if (!kPlain && red.tiles->enabled) classify_tiles<kSolve32>(a, *red.tiles);
                 if (!diffusion<kSolve32, kResident>(a, red, st.cur, dt, d)) return false;
                 good = d.ok;
                 out.cg_iterations = d.it;
@@ -2677,7 +2795,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     }
     __shared__ Tiles tiles;
     // (a tape takes the whole solution plane of every step)
-    init_tiles(tiles, a, kRun && !kSolve32 && !args.tape);
+    init_tiles(tiles, a, kRun && !args.tape);
     __syncthreads();
     Red red(a, &clk);
     red.pipe_ptr = &pipe;
@@ -2739,7 +2857,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     if (args.mode == kModePropose) {
         double change;
         bool mixbad, simplexbad;
-        if (!phase_propose<!kSolve32 && !kPlain>(a, red, st.cur, args.dt, change, mixbad, simplexbad)) return;
+        if (!phase_propose<!kPlain>(a, red, st.cur, args.dt, change, mixbad, simplexbad)) return;
         if (leader) {
             ctl->out[0] = change;
             ctl->iout[0] = mixbad;
@@ -2889,7 +3007,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs& args) {
         }
         __syncthreads();
         const Dom a{sP, sB, I->maps, args.use_tma, bid, nblk, gctl, gpart, 0, 0, 0, 0, 0, 0, 0};
-        init_tiles(tiles, a, !kSolve32);
+        init_tiles(tiles, a, true);
         __syncthreads();
         Red red(a, &clk, reductions);
         red.pipe_ptr = &pipe;

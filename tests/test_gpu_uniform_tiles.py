@@ -108,3 +108,27 @@ def test_batch_bitwise(gpu_lib, port, group):
         po, co, muo, so, _ = _oracle(port, w, n, 8, group)
         assert s.time == so.time
         assert np.array_equal(phi, po) and np.array_equal(c, co) and np.array_equal(mu, muo)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "mixed_solve", "mixed_propose"])
+@pytest.mark.parametrize("nx,ny,warps,front,dscale,variant", CASES)
+def test_mixed_forms_equal_dense_runs(gpu_lib, monkeypatch, nx, ny, warps, front, dscale, variant, precision):
+    """The mixed forms have no oracle: a staged run, which leaves uniform tiles
+    out, against an unstaged one, which does not look for them."""
+    import pearl_gpu
+
+    w = _workload(nx, ny, front, dscale, variant)
+    monkeypatch.setenv("PEARL_GPU_TILE_WARPS", str(warps))
+    monkeypatch.setenv("PEARL_GPU_GRID", "7")
+    got = []
+    for tma in ("1", "0"):
+        monkeypatch.setenv("PEARL_GPU_TMA", tma)
+        with pearl_gpu.Context(w.params, nx, ny) as ctx:
+            ctx.set_precision(precision)
+            ctx.upload(w.phi, w.carbon, w.mu, w.scalars)
+            reports = [ctx.run(k) for k in (2, 4)]
+            got.append((ctx.download(), [(r.steps, r.cg_total, r.last.linear_residual) for r in reports]))
+    (a, ra), (b, rb) = got
+    assert ra == rb and sum(r[0] for r in ra) == 6
+    assert (a[3].time, a[3].rejected) == (b[3].time, b[3].rejected)
+    assert all(np.array_equal(x, y) for x, y in zip(a[:3], b[:3]))
