@@ -2431,25 +2431,25 @@ __device__ bool maybe_shift(const Dom& a, Red& red, StepState& st, int& rows_out
 
 // ------------------------------------------------------------------ initialisation
 // Interface-only energy density of one cell (interface_energy_only,
-// pearl_serial.cpp:822-842), without the final dx*dy.
+// pearl_serial.cpp:822-842), without the final dx*dy.  Most cells of a sharp
+// domain equal their neighbours: a face whose three products vanish adds +0 to
+// the sum and is left out, so a warp away from the interfaces divides nowhere.
+__device__ __forceinline__ double interface_face_energy(const DevParams& P, double t, const Phi3& q, const Phi3& n,
+                                                        double d, double rd) {
+    const double z0 = q.a * n.t - n.a * q.t, z1 = q.a * n.g - n.a * q.g, z2 = q.t * n.g - n.t * q.g;
+    if (z0 == 0 && z1 == 0 && z2 == 0) return t;
+    double z = div_by(P, z0, d, rd);
+    t += P.eps_sigma * z * z;
+    z = div_by(P, z1, d, rd);
+    t += P.eps_sigma * z * z;
+    z = div_by(P, z2, d, rd);
+    return t + P.eps_sigma * z * z;
+}
 __device__ __forceinline__ double interface_energy_cell(const DevParams& P, const Phi3& q, const Phi3& e,
                                                         const Phi3& n, bool has_n) {
     double t = P.obs * (q.a * q.t + q.a * q.g + q.t * q.g) + P.tr * q.a * q.t * q.g;
-    double z = div_by(P, q.a * e.t - e.a * q.t, P.dx, P.r_dx);
-    t += P.eps_sigma * z * z;
-    z = div_by(P, q.a * e.g - e.a * q.g, P.dx, P.r_dx);
-    t += P.eps_sigma * z * z;
-    z = div_by(P, q.t * e.g - e.t * q.g, P.dx, P.r_dx);
-    t += P.eps_sigma * z * z;
-    if (has_n) {
-        z = div_by(P, q.a * n.t - n.a * q.t, P.dy, P.r_dy);
-        t += P.eps_sigma * z * z;
-        z = div_by(P, q.a * n.g - n.a * q.g, P.dy, P.r_dy);
-        t += P.eps_sigma * z * z;
-        z = div_by(P, q.t * n.g - n.t * q.g, P.dy, P.r_dy);
-        t += P.eps_sigma * z * z;
-    }
-    return t;
+    t = interface_face_energy(P, t, q, e, P.dx, P.r_dx);
+    return has_n ? interface_face_energy(P, t, q, n, P.dy, P.r_dy) : t;
 }
 
 // Interface-only energy of state set `s` plus its phase-fraction sums.
@@ -2511,13 +2511,15 @@ __device__ bool phase_smooth_force(const Dom& a, Red& red, int cur, double& forc
                 if ((dir == 2 && y == 0) || (dir == 3 && y == P.ny - 1)) continue;
                 const size_t j = dir == 0 ? iw : (dir == 1 ? ie : (dir == 2 ? is : in));
                 const double n[3] = {ph[0][j], ph[1][j], ph[2][j]};
-                const double d2 = dir < 2 ? P.dx2 : P.dy2;
-        const double rd2 = dir < 2 ? P.r_dx2 : P.r_dy2;
+                const double x[3] = {q[0] * n[1] - n[0] * q[1], q[0] * n[2] - n[0] * q[2], q[1] * n[2] - n[1] * q[2]};
+                // a face without a gradient adds +-0 to forces that are never -0
+                if (x[0] == 0 && x[1] == 0 && x[2] == 0) continue;
+                const double d2 = dir < 2 ? P.dx2 : P.dy2, rd2 = dir < 2 ? P.r_dx2 : P.r_dy2;
 #pragma unroll
                 for (int aa = 0; aa < 3; ++aa)
 #pragma unroll
                     for (int b = aa + 1; b < 3; ++b) {
-                        const double w = div_by(P, P.two_eps_sigma * (q[aa] * n[b] - n[aa] * q[b]), d2, rd2);
+                        const double w = div_by(P, P.two_eps_sigma * x[aa + b - 1], d2, rd2);
                         f[aa] += w * n[b];
                         f[b] -= w * n[aa];
                     }
@@ -2537,35 +2539,53 @@ __device__ bool phase_smooth_force(const Dom& a, Red& red, int cur, double& forc
     return true;
 }
 
-// Backtracking trial of smooth_interface_only (pearl_serial.cpp:925-933):
-// trial phi = project(phi - scale*force) into set cur^1.
-// Reduction: {max |dphi|, simplex failed}.
-__device__ bool phase_smooth_trial(const Dom& a, Red& red, int cur, double scale, double& change, bool& bad) {
+// Backtracking trial of smooth_interface_only (pearl_serial.cpp:925-933) with
+// its energy: trial phi = project(phi - scale*force) into set cur^1, and the
+// interface energy of that trial in the same pass, the trial of the cells
+// beyond the pair formed again instead of read after a grid barrier.
+// Reduction: {energy sum, max |dphi|, simplex failed}.
+__device__ bool phase_smooth_trial(const Dom& a, Red& red, int cur, double scale, double& change, bool& bad,
+                                   double& energy) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
     const double* const* ph = B.phi[cur];
     double* const* tp = B.phi[cur ^ 1];
-    double vch = 0, vbad = 0;
+    double ven = 0, vch = 0, vbad = 0;
+    const auto trial = [&](size_t i, Phi3& q) {
+        q = load_phi(ph, i);
+        Phi3 z{q.a - scale * B.x[i], q.t - scale * B.r[i], q.g - scale * B.z[i]};
+        const bool ok = isfinite(z.a) && isfinite(z.t) && isfinite(z.g) && project_simplex(P, z.a, z.t, z.g);
+        if (!ok) vbad = 1;
+        return z;
+    };
+    const auto own = [&](size_t i) {
+        Phi3 q;
+        const Phi3 z = trial(i, q);
+        vch = fmax(vch, fabs(z.a - q.a));
+        vch = fmax(vch, fabs(z.t - q.t));
+        vch = fmax(vch, fabs(z.g - q.g));
+        tp[0][i] = z.a;
+        tp[1][i] = z.t;
+        tp[2][i] = z.g;
+        return z;
+    };
     FOR_TILES(P) {
         const Pair c = pair_of(P, t);
-        for (int k = 0; k < 2; ++k) {
-            if (!(k ? c.v1 : c.v0)) continue;
-            const size_t i = k ? c.i1 : c.i0;
-            const double q0 = ph[0][i], q1 = ph[1][i], q2 = ph[2][i];
-            double z0 = q0 - scale * B.x[i], z1 = q1 - scale * B.r[i], z2 = q2 - scale * B.z[i];
-            if (!(isfinite(z0) && isfinite(z1) && isfinite(z2)) || !project_simplex(P, z0, z1, z2)) vbad = 1;
-            vch = fmax(vch, fabs(z0 - q0));
-            vch = fmax(vch, fabs(z1 - q1));
-            vch = fmax(vch, fabs(z2 - q2));
-            tp[0][i] = z0;
-            tp[1][i] = z1;
-            tp[2][i] = z2;
+        if (!c.v0) continue;
+        Phi3 q;
+        const Phi3 lower = own(c.i0), none{0, 0, 0};
+        const Phi3 upper = c.v1 ? own(c.i1) : none;
+        ven += interface_energy_cell(P, lower, trial(c.ie0, q), upper, c.v1);
+        if (c.v1) {
+            const bool has_n = c.y0 + 1 < P.ny - 1;
+            ven += interface_energy_cell(P, upper, trial(c.ie1, q), has_n ? trial(c.in1, q) : none, has_n);
         }
     }
-    double v[2] = {vch, vbad};
-    if (!red.reduce<2>(v, OPS2(kMax, kMax), kTagSmooth)) return false;
-    change = v[0];
-    bad = v[1] != 0;
+    double v[3] = {ven, vch, vbad};
+    if (!red.reduce<3>(v, OPS3(kSum, kMax, kMax), kTagSmooth)) return false;
+    energy = v[0] * P.dx * P.dy;
+    change = v[1];
+    bad = v[2] != 0;
     return true;
 }
 
@@ -2607,13 +2627,11 @@ __device__ bool smooth(const Dom& a, Red& red, StepState& st, double* rep) {
         double new_energy = previous, actual_change = 0;
         for (int backtrack = 0; backtrack < 24 && !accepted; ++backtrack) {
             bool bad;
-            if (!phase_smooth_trial(a, red, st.cur, scale, actual_change, bad)) return false;
+            if (!phase_smooth_trial(a, red, st.cur, scale, actual_change, bad, new_energy)) return false;
             if (bad) {
                 set_error(a, PEARL_ERR_SIMPLEX, 0);
                 return false;
             }
-            double f3[3];
-            if (!phase_interface_energy(a, red, st.cur ^ 1, new_energy, f3)) return false;
             double big = 1.0;
             if (big < fabs(previous)) big = fabs(previous);
             if (big < fabs(e_init)) big = fabs(e_init);
