@@ -30,6 +30,8 @@ struct pearl_gpu_batch {
     Ctl* d_group_ctl = nullptr;
     double* d_group_part = nullptr;
     int per_sm = 0, sms = 0, grid = 0, group_blocks = 0, ngroups = 0;  // group_blocks -1: sized per instance
+    const void* prepared = nullptr;  // kernel of the last launch, and its staging
+    bool prepared_tma = false;
     double pass_overhead_tiles = 4;  // sized groups: fixed cost of a pass, in tiles of one block
     bool use_tma = true;      // TMA staging in use (needs the 32x16 tile)
     bool tma_capable = true;  // tensor maps of every instance encoded and the shared memory granted
@@ -235,6 +237,29 @@ const void* batch_kernel(bool solve32, bool fast_div) {
     return kernels[solve32][fast_div];
 }
 
+// The kernel of the batch's instances: the mixed form's inner solve has one of
+// its own (all instances share one precision, pearl_gpu_batch_set_precision),
+// and one instance whose divisors need the general division decides for all.
+const void* batch_kernel_of(const pearl_gpu_batch* b) {
+    bool solve32 = false, fast = true;
+    for (auto* c : b->inst) {
+        solve32 = solve32 || c->P.mixed_cg;
+        fast = fast && c->P.fast_div;
+    }
+    return batch_kernel(solve32, fast);
+}
+
+// Prepares `kernel` where the last launch was not of it; the whole grid must be co-resident.
+cudaError_t batch_prepare(pearl_gpu_batch* b, const void* kernel, bool tma) {
+    if (b->prepared == kernel && b->prepared_tma == tma) return cudaSuccess;
+    constexpr TileGeometry g = tile_geometry(8);
+    const cudaError_t e = prepare_kernel(kernel, g.threads, tma ? g.tma_smem_bytes : 0, b->per_sm * b->sms, b->sms);
+    if (e != cudaSuccess) return e;
+    b->prepared = kernel;
+    b->prepared_tma = tma;
+    return cudaSuccess;
+}
+
 int batch_launch(pearl_gpu_batch* b, const pearl_run_limits& L) {
     const NvtxRange range("pearl_gpu batch run");
     PB_CUDA(b, cudaSetDevice(b->device));
@@ -252,14 +277,8 @@ int batch_launch(pearl_gpu_batch* b, const pearl_run_limits& L) {
     void* kargs[] = {&args};
     PB_CUDA(b, cudaEventRecord(b->ev0, b->stream));
     constexpr TileGeometry g = tile_geometry(8);
-    // the mixed form's inner solve runs in a kernel of its own (all instances
-    // of a batch share one precision, pearl_gpu_batch_set_precision)
-    bool solve32 = false;
-    for (auto* c : b->inst) solve32 = solve32 || c->P.mixed_cg;
-    // one instance whose divisors need the general division decides for all
-    bool fast = true;
-    for (auto* c : b->inst) fast = fast && c->P.fast_div;
-    const void* kernel = batch_kernel(solve32, fast);
+    const void* const kernel = batch_kernel_of(b);
+    PB_CUDA(b, batch_prepare(b, kernel, b->use_tma));
     PB_CUDA(b, cudaLaunchCooperativeKernel(kernel, dim3(b->grid), dim3(g.threads), kargs,
                                            b->use_tma ? g.tma_smem_bytes : 0, b->stream));
     b->launches++;
@@ -319,7 +338,7 @@ int pearl_gpu_batch_create(int n, const pearl_params* params, const int* nx, con
     std::memset(b->h_ctls, 0, sizeof(Ctl) * n);
     bool tma = true;
     for (int i = 0; i < n; ++i) {
-        const int rc = pearl_gpu_create(&params[i], nx[i], ny[i], device, &b->inst[i]);
+        const int rc = create_context(&params[i], nx[i], ny[i], device, false, &b->inst[i]);
         if (rc) return bail(rc);
         pearl_gpu_ctx* c = b->inst[i];
         set_geometry(c, 8);  // the batch kernel runs 256-thread blocks, two per SM
@@ -333,22 +352,13 @@ int pearl_gpu_batch_create(int n, const pearl_params* params, const int* nx, con
     if (cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess)
         return bail(PEARL_ERR_CUDA);
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device);
-    const void* kernels[4];
-    for (int k = 0; k < 4; ++k) kernels[k] = batch_kernel(k & 1, k & 2);
-    for (const void* k : kernels)
-        if (tma && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)tile_geometry(8).tma_smem_bytes) != cudaSuccess)
-            tma = false;
-    b->per_sm = 1 << 30;
-    for (const void* k : kernels) {
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, tile_geometry(8).threads,
-                                                          tma ? tile_geometry(8).tma_smem_bytes : 0) != cudaSuccess ||
-            n < 1)
-            return bail(PEARL_ERR_CUDA);
-        b->per_sm = std::min(b->per_sm, n);
-    }
+    constexpr TileGeometry g = tile_geometry(8);
+    b->per_sm = g.min_blocks;  // (checked for each kernel at its first launch)
     b->tma_capable = tma;
+    if (tma && batch_prepare(b, batch_kernel_of(b), true) != cudaSuccess) {
+        cudaGetLastError();
+        b->tma_capable = tma = false;
+    }
     const int rc = batch_configure(b, group_blocks > 0 ? group_blocks : PEARL_BATCH_SIZED_GROUPS, tma, 0);
     if (rc) return bail(rc);
     *out = b;

@@ -89,9 +89,38 @@ const void* plain_step_kernel(int grid, int sms) {
     return grid <= sms ? (const void*)plain_wide::pearl_kernel : (const void*)plain::pearl_kernel;
 }
 
+cudaError_t prepare_kernel(const void* kernel, int threads, size_t smem, int grid, int sms) {
+    if (smem > 0) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    int n = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    return (long long)n * sms >= grid ? cudaSuccess : cudaErrorCooperativeLaunchTooLarge;
+}
+
+namespace {
+// The kernel of a launch of this context, prepared on its first use: a kernel
+// that is never launched is never loaded.
+const void* launch_kernel(pearl_gpu_ctx* ctx, StepKernel kind, bool tma, cudaError_t& e) {
+    const bool fast = ctx->P.fast_div != 0, plain = kind == kStepRun && !tma && ctx->warps == 8 && fast;
+    const void* kernel = plain ? plain_step_kernel(ctx->grid, ctx->sms) : step_kernel(ctx->warps, kind, fast);
+    const unsigned bit = plain ? 1u << 12 : 1u << (4 * kind + 2 * (int)fast + (int)tma);
+    e = cudaSuccess;
+    if (!(ctx->prepared & bit)) {
+        const TileGeometry g = tile_geometry(ctx->warps);
+        e = prepare_kernel(kernel, g.threads, tma ? g.tma_smem_bytes : 0, ctx->grid, ctx->sms);
+        if (e == cudaSuccess) ctx->prepared |= bit;
+    }
+    return kernel;
+}
+}  // namespace
+
 void set_geometry(pearl_gpu_ctx* ctx, int warps) {
     if (ctx->warps == warps) return;
     ctx->warps = warps;
+    ctx->prepared = 0;
     set_tile_shape(ctx, ctx->P.warps_x_log2);
     if (ctx->use_tma && !build_tensor_maps(ctx)) ctx->use_tma = false;
 }
@@ -217,8 +246,9 @@ int launch(pearl_gpu_ctx* ctx, KArgs& args) {
     if (tma) std::memcpy(args.maps, ctx->maps, sizeof ctx->maps);
     const TileGeometry g = tile_geometry(ctx->warps);
     const StepKernel kind = args.mode != kModeRun ? kStepModes : ctx->P.mixed_cg ? kStepRunMixed : kStepRun;
-    const void* kernel = step_kernel(ctx->warps, kind, ctx->P.fast_div != 0);
-    if (kind == kStepRun && !tma && ctx->warps == 8 && ctx->P.fast_div) kernel = plain_step_kernel(ctx->grid, ctx->sms);
+    cudaError_t prepared;
+    const void* const kernel = launch_kernel(ctx, kind, tma, prepared);
+    PG_CUDA(ctx, prepared);
     PG_CUDA(ctx, cudaLaunchCooperativeKernel(kernel, dim3(ctx->grid),
                                              dim3(g.threads), kargs,
                                              tma ? g.tma_smem_bytes : 0, ctx->stream));
@@ -596,6 +626,13 @@ const char* pearl_gpu_status_string(int status) {
 const char* pearl_gpu_last_error(const pearl_gpu_ctx* ctx) { return ctx ? ctx->error.c_str() : "null context"; }
 
 int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pearl_gpu_ctx** out) {
+    return create_context(params, nx, ny, device, true, out);
+}
+
+}  // extern "C"
+
+int pearl_gpu::create_context(const pearl_params* params, int nx, int ny, int device, bool prepare,
+                              pearl_gpu_ctx** out) {
     if (!out) return PEARL_ERR_INVALID_ARGUMENT;
     *out = nullptr;
     if (!params || nx < 3 || ny < 2 || !valid_params(params)) return PEARL_ERR_INVALID_ARGUMENT;
@@ -637,26 +674,10 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     const char* tma_env = std::getenv("PEARL_GPU_TMA");
     ctx->use_tma = ctx->P.warps_x_log2 == 0 && !(tma_env && std::atoi(tma_env) == 0);
     const TileGeometry geom = tile_geometry(ctx->warps);
-    // every kernel of the block shape (parameters and precision may change later)
-    // gets the stage buffers; the grid fits the residency of all
-    const void* kernels[6];
-    for (int k = 0; k < 6; ++k) kernels[k] = step_kernel(ctx->warps, (StepKernel)(k / 2), k & 1);
     ctx->sms = sms;
-    for (const void* k : kernels)
-        if (ctx->use_tma && cudaFuncSetAttribute(k,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)geom.tma_smem_bytes) != cudaSuccess)
-            ctx->use_tma = false;
-    int per_sm = 1 << 30;
-    for (const void* k : kernels) {
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, geom.threads,
-                                                          ctx->use_tma ? geom.tma_smem_bytes : 0) != cudaSuccess ||
-            n < 1)
-            return bail(PEARL_ERR_CUDA);
-        per_sm = std::min(per_sm, n);
-    }
-    ctx->grid = std::max(1, std::min(per_sm * sms, ctx->P.ntiles));
+    // the blocks per SM that every kernel of the shape is compiled for (checked
+    // when a kernel is first launched)
+    ctx->grid = std::max(1, std::min(geom.min_blocks * sms, ctx->P.ntiles));
     // PEARL_GPU_GRID caps the block count (the grid-size sweeps of small domains)
     if (const char* e = std::getenv("PEARL_GPU_GRID"))
         if (std::atoi(e) > 0) ctx->grid = std::min(ctx->grid, std::atoi(e));
@@ -667,6 +688,16 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     // 1024x2048, 13.8 tiles, 0.497 against 0.601; 256x512 0.0947 against
     // 0.0733).  PEARL_GPU_TMA=1 stages whatever the size, =0 never.
     ctx->stage_tma = ctx->use_tma && ((tma_env && std::atoi(tma_env) != 0) || ctx->P.ntiles >= 6LL * ctx->grid);
+    if (prepare) {
+        cudaError_t e;
+        launch_kernel(ctx, kStepRun, ctx->stage_tma, e);
+        if (e != cudaSuccess && ctx->stage_tma) {  // no stage buffers to be had: the kernels read the planes directly
+            cudaGetLastError();
+            ctx->use_tma = ctx->stage_tma = false;
+            launch_kernel(ctx, kStepRun, false, e);
+        }
+        if (e != cudaSuccess) return bail(PEARL_ERR_CUDA);
+    }
     // state: 2 x (3 phi + c + mu); work: K chi icpt diag x r z p0 p1 Ap  -> 20 planes
     const size_t pe = plane_elems(ctx);
     const int nplanes = 22;
@@ -711,6 +742,8 @@ int pearl_gpu_create(const pearl_params* params, int nx, int ny, int device, pea
     *out = ctx;
     return PEARL_OK;
 }
+
+extern "C" {
 
 void pearl_gpu_destroy(pearl_gpu_ctx* ctx) {
     if (!ctx) return;

@@ -38,6 +38,7 @@ struct pearl_gpu_ctx {
     size_t stage_elems = 0;
     int grid = 0;
     int sms = 0;  // of the device
+    unsigned prepared = 0;  // kernels that this context has launched (launch_kernel)
     long long launches = 0;
     double last_ms = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -69,6 +70,11 @@ const void* step_kernel(int warps, StepKernel kind, bool fast_div);
 // The step loop of a domain of 8-warp blocks that does not stage: compiled for
 // one block per SM where the grid allows that, else for two.
 const void* plain_step_kernel(int grid, int sms);
+// Shared memory opt-in of a kernel, and the check that `grid` blocks of it are co-resident.
+cudaError_t prepare_kernel(const void* kernel, int threads, size_t smem, int grid, int sms);
+// pearl_gpu_create; prepare: with the step kernel of a context of its own (an
+// instance of a batch runs the batch's kernel).
+int create_context(const pearl_params* params, int nx, int ny, int device, bool prepare, pearl_gpu_ctx** out);
 // Gives the context the kernels of another block shape (tile counts and TMA
 // boxes follow); its own launch grid is kept.
 void set_geometry(pearl_gpu_ctx* ctx, int warps);

@@ -131,15 +131,14 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
     B.part = scratch + kNoAllocPlanes * (size_t)kNoAllocMaxCells;
     B.ctl = reinterpret_cast<Ctl*>(B.part + (size_t)2 * kNoAllocMaxBlocks * kMaxRed);
 
-    int sms = 0, per_sm = 0;
+    int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return PEARL_ERR_CUDA;
     const void* const kernel =
         ctx.P.fast_div ? plain_step_kernel(ctx.P.ntiles, sms) : step_kernel(8, kStepRun, false);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tile_geometry(8).threads, 0) !=
-            cudaSuccess ||
-        per_sm < 1)
-        return PEARL_ERR_CUDA;
-    const int grid = std::max(1, std::min(std::min(per_sm * sms, ctx.P.ntiles), kNoAllocMaxBlocks));
+    // the blocks per SM that the kernels are compiled for; a device that cannot hold
+    // them refuses the cooperative launch
+    const int grid =
+        std::max(1, std::min(std::min(tile_geometry(8).min_blocks * sms, ctx.P.ntiles), kNoAllocMaxBlocks));
 
     // The scratch keeps the previous call's contents: reset the control block
     // (status, barrier counter, cached energies) before the launch.
