@@ -402,6 +402,7 @@ int stage_grid(const pearl_gpu_ctx* ctx) {
     return (int)std::max(1LL, std::min<long long>((n + 255) / 256, 148LL * 16));
 }
 
+// (the caller waits for the stream before it returns: the host's buffers are read until then)
 int upload_set(pearl_gpu_ctx* ctx, int set, const double* phi, const double* carbon, const double* mu) {
     const NvtxRange range("pearl_gpu upload");
     if (int rc = ensure_stage(ctx)) return rc;
@@ -416,7 +417,6 @@ int upload_set(pearl_gpu_ctx* ctx, int set, const double* phi, const double* car
         ctx->B.phi[set][2], carbon ? ctx->B.c[set] : nullptr, mu ? ctx->B.mu[set] : nullptr);
     ctx->launches++;
     PG_CUDA(ctx, cudaGetLastError());
-    PG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return PEARL_OK;
 }
 
@@ -1099,6 +1099,7 @@ int pearl_gpu_upload_trial_phi(pearl_gpu_ctx* ctx, const double* phi) {
     if (!ctx || !phi) return PEARL_ERR_INVALID_ARGUMENT;
     int rc = upload_set(ctx, ctx->h_ctl->cur ^ 1, phi, nullptr, nullptr);
     if (rc) return rc;
+    PG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     KArgs a{};
     a.mode = kModeMix;
     rc = launch(ctx, a);

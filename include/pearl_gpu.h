@@ -376,7 +376,9 @@ int pearl_gpu_adjoint_gradient(pearl_gpu_ctx* ctx, long long nsteps, int checkpo
  * the groups have per-instance sizes instead, chosen so that the slowest group
  * finishes soonest under a model of a pass's cost (powers of two up to the
  * grid, or an equal share of the grid per instance): small instances share
- * groups of a few blocks, large ones get many.  Every instance follows exactly the path of a
+ * groups of a few blocks, large ones get many.  With two blocks or more
+ * an instance, the sizes follow the uploaded states: an instance gets blocks in
+ * proportion to the part of it that is not uniform austenite.  Every instance follows exactly the path of a
  * pearl_gpu_ctx (same kernels, same reduction order for the same group size),
  * so it is main's loop (pearl_serial.cpp:2296-2306) run once per instance.
  * No counterpart in the reference, which runs one case per process. */
