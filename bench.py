@@ -153,6 +153,17 @@ def phase_hbm_fracs(phase_ms: dict, phase_n: dict, cells: int, peak_gbs: float) 
     return out
 
 
+def non_uniform_cells(phi, carbon, mu) -> int:
+    """Cells that differ from the reference cell ahead of the front (the kernels'
+    reference for uniform tiles)."""
+    ny, nx = mu.shape
+    y, x = ny - 1 - ny // 16, nx // 2
+    same = (mu == mu[y, x]) & (carbon == carbon[y, x])
+    for a in range(3):
+        same &= phi[..., a] == phi[y, x, a]
+    return int(same.size - same.sum())
+
+
 def ncu_traffic_per_cell():
     """DRAM bytes per cell-update of pearl_kernel from the committed ncu summary, or None."""
     p = ROOT / "profiles" / "pearl_kernel_fp64_plain_large.md"
@@ -385,8 +396,11 @@ def gpu_arm(args, rank: int, world: int, dist) -> None:
     assert rep.steps == args.steps, "run stopped early"
     value, t_max = replica_throughput(dist, float(w.cells * rep.steps), elapsed, "cuda")
 
-    # roofline of the persistent kernel: algorithmic bytes of its launch over its event time
-    algo_bytes = w.cells * (80.0 * rep.steps + 64.0 * rep.cg_total)
+    # roofline of the persistent kernel: algorithmic bytes of its launch over its
+    # event time, of the cells that have work of their own (cells equal to the
+    # austenite ahead of the front are computed once and not moved)
+    dense_cells = non_uniform_cells(*ctx.download()[:3])
+    algo_bytes = dense_cells * (80.0 * rep.steps + 64.0 * rep.cg_total)
     achieved = algo_bytes / (kernel_ms / 1e3) / 1e9
     peak, peak_kind = measured_peak()
     tpc = ncu_traffic_per_cell()
@@ -435,11 +449,12 @@ def gpu_arm(args, rank: int, world: int, dist) -> None:
                          "spec_gbs": SPEC_HBM_GBS, "frac_of_spec": achieved / SPEC_HBM_GBS,
                          "peak_source": f"{peak_kind} HBM copy bandwidth",
                          "kernel": "pearl_kernel (persistent FP64 step)",
-                         # 148 on B200: one 512-thread block per SM (32x32 tiles); 296: two 256-thread blocks
+                         # 296 on B200: two 256-thread blocks per SM (32x16 tiles); 148: one 512-thread block
                          "grid_blocks": ctx.stats()["grid"],
                          "algorithmic_bytes_per_launch": algo_bytes, "cg_iterations": rep.cg_total,
+                         "non_uniform_cells": dense_cells,
                          "rejected_attempts": rejected, "phase_ms": phase_ms, "phase_count": phase_n,
-                         "phase_hbm_frac": phase_hbm_fracs(phase_ms, phase_n, w.cells, peak),
+                         "phase_hbm_frac": phase_hbm_fracs(phase_ms, phase_n, dense_cells, peak),
                          "phase_bytes_per_cell": PHASE_BYTES},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": bytes_state / m,
@@ -583,7 +598,8 @@ def sweep_arm(args, rank: int, world: int, dist) -> None:
                          "frac": achieved / peak, "traffic": None,
                          "spec_gbs": SPEC_HBM_GBS, "frac_of_spec": achieved / SPEC_HBM_GBS,
                          "peak_source": f"{peak_kind} HBM copy bandwidth",
-                         "kernel": "pearl_batch_kernel (persistent FP64 step, block groups)",
+                         "kernel": "pearl_batch_kernel (persistent FP64 step, block groups; bytes of every cell, "
+                                   "uniform tiles move next to none)",
                          "algorithmic_bytes_per_launch": algo_bytes,
                          "rejected_attempts": int(sum(rejected)),
                          "cg_per_step": sum(r.cg_total for r in reps) / max(1, sum(steps)),
