@@ -18,9 +18,13 @@
 // kTileY warps of a block stack 2 x kTileY rows.  This file is compiled once
 // per block shape (PEARL_TILE_WARPS = 8: 32x16 tiles, two 256-thread blocks
 // per SM; 16: 32x32 tiles, one 512-thread block per SM), into namespaces g8
-// and g16.  The two cells of a thread share their vertical neighbour loads.
+// and g16; once more each with the general division, for parameters whose constants
+// the two-operation one is not proved for (g8_div, g16_div); and without the
+// staging, for domains with few tiles a block (plain, plain_wide).  The two cells of a
+// thread share their vertical neighbour loads.
 // Each phase's input fields are staged per tile by 2-D TMA copies into shared
-// memory through an mbarrier pipeline (`sweep`).
+// memory through an mbarrier pipeline (`sweep`), which passes over tiles that
+// are uniform; the plain kernels read them from global memory.
 //
 // This file also holds the batched kernel (block groups running independent
 // instances), the self-test kernels, and, through pearl_adjoint.cuh, the
