@@ -85,7 +85,8 @@ const void* step_kernel(int warps, StepKernel kind, bool fast_div) {
     return kernels[warps == 16][kind][fast_div];
 }
 
-const void* plain_step_kernel(int grid, int sms) {
+const void* plain_step_kernel(int grid, int sms, bool held) {
+    if (held) return (const void*)plain_held::pearl_kernel;
     return grid <= sms ? (const void*)plain_wide::pearl_kernel : (const void*)plain::pearl_kernel;
 }
 
@@ -103,14 +104,17 @@ cudaError_t prepare_kernel(const void* kernel, int threads, size_t smem, int gri
 namespace {
 // The kernel of a launch of this context, prepared on its first use: a kernel
 // that is never launched is never loaded.
-const void* launch_kernel(pearl_gpu_ctx* ctx, StepKernel kind, bool tma, cudaError_t& e) {
+const void* launch_kernel(pearl_gpu_ctx* ctx, StepKernel kind, bool tma, cudaError_t& e, int& held, size_t& smem) {
     const bool fast = ctx->P.fast_div != 0, plain = kind == kStepRun && !tma && ctx->warps == 8 && fast;
-    const void* kernel = plain ? plain_step_kernel(ctx->grid, ctx->sms) : step_kernel(ctx->warps, kind, fast);
+    held = plain ? held_fields(ctx->P.ntiles, ctx->grid) : 0;
+    const void* kernel = plain ? plain_step_kernel(ctx->grid, ctx->sms, held) : step_kernel(ctx->warps, kind, fast);
     const unsigned bit = plain ? 1u << 12 : 1u << (4 * kind + 2 * (int)fast + (int)tma);
+    const TileGeometry g = tile_geometry(ctx->warps);
+    smem = tma ? g.tma_smem_bytes : held ? held_bytes(ctx->P.ntiles, ctx->grid, g.threads) : 0;
     e = cudaSuccess;
     if (!(ctx->prepared & bit)) {
-        const TileGeometry g = tile_geometry(ctx->warps);
-        e = prepare_kernel(kernel, g.threads, tma ? g.tma_smem_bytes : 0, ctx->grid, ctx->sms);
+        // (the most that any domain holds: the attribute is the kernel's, not the context's)
+        e = prepare_kernel(kernel, g.threads, held ? kHeldMaxBytes : smem, ctx->grid, ctx->sms);
         if (e == cudaSuccess) ctx->prepared |= bit;
     }
     return kernel;
@@ -245,13 +249,13 @@ int launch(pearl_gpu_ctx* ctx, KArgs& args) {
     args.use_tma = tma ? 1 : 0;
     if (tma) std::memcpy(args.maps, ctx->maps, sizeof ctx->maps);
     const TileGeometry g = tile_geometry(ctx->warps);
+    size_t smem;
     const StepKernel kind = args.mode != kModeRun ? kStepModes : ctx->P.mixed_cg ? kStepRunMixed : kStepRun;
     cudaError_t prepared;
-    const void* const kernel = launch_kernel(ctx, kind, tma, prepared);
+    const void* const kernel = launch_kernel(ctx, kind, tma, prepared, args.held_fields, smem);
     PG_CUDA(ctx, prepared);
     PG_CUDA(ctx, cudaLaunchCooperativeKernel(kernel, dim3(ctx->grid),
-                                             dim3(g.threads), kargs,
-                                             tma ? g.tma_smem_bytes : 0, ctx->stream));
+                                             dim3(g.threads), kargs, smem, ctx->stream));
     ctx->launches++;
     PG_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     rc = pull_ctl(ctx);
@@ -690,11 +694,13 @@ int pearl_gpu::create_context(const pearl_params* params, int nx, int ny, int de
     ctx->stage_tma = ctx->use_tma && ((tma_env && std::atoi(tma_env) != 0) || ctx->P.ntiles >= 6LL * ctx->grid);
     if (prepare) {
         cudaError_t e;
-        launch_kernel(ctx, kStepRun, ctx->stage_tma, e);
+        int held;
+        size_t smem;
+        launch_kernel(ctx, kStepRun, ctx->stage_tma, e, held, smem);
         if (e != cudaSuccess && ctx->stage_tma) {  // no stage buffers to be had: the kernels read the planes directly
             cudaGetLastError();
             ctx->use_tma = ctx->stage_tma = false;
-            launch_kernel(ctx, kStepRun, false, e);
+            launch_kernel(ctx, kStepRun, false, e, held, smem);
         }
         if (e != cudaSuccess) return bail(PEARL_ERR_CUDA);
     }

@@ -18,8 +18,9 @@
 // The device code is compiled for two block shapes (PEARL_TILE_WARPS) and two
 // ways of dividing by the formulas' constants (PEARL_FAST_DIV, see div_const),
 // each in a namespace of its own.  PEARL_PLAIN adds the step loop of domains that
-// do not stage (8 warps; 2: of those with at most one block per SM), without the
-// staging pipeline's code and registers.
+// do not stage (8 warps; 2: of those with at most one block per SM; 3: of those
+// whose solve keeps its values in shared memory), without the staging pipeline's
+// code and registers.
 #ifndef PEARL_PLAIN
 #define PEARL_PLAIN 0
 #endif
@@ -33,6 +34,8 @@
 #define PEARL_GEOM_NS plain
 #elif PEARL_PLAIN == 2
 #define PEARL_GEOM_NS plain_wide
+#elif PEARL_PLAIN == 3
+#define PEARL_GEOM_NS plain_held
 #elif PEARL_TILE_WARPS == 16
 #define PEARL_GEOM_NS PEARL_NS_(g16, PEARL_FAST_DIV)
 #elif PEARL_TILE_WARPS == 8
@@ -325,7 +328,7 @@ constexpr size_t kTmaSmemBytes = kGeom.tma_smem_bytes;
 // The wide plain kernel has an SM to a block: 255 registers a thread, enough to
 // work on both cells of a thread at once (kCellUnroll) where the others take one
 // after the other.
-constexpr bool kPlain = PEARL_PLAIN != 0;
+constexpr bool kPlain = PEARL_PLAIN != 0, kHeldSolve = PEARL_PLAIN == 3;
 constexpr int kMinBlocks = PEARL_PLAIN == 2 ? 1 : kGeom.min_blocks;
 constexpr int kCellUnroll = PEARL_PLAIN == 2 ? 2 : 1;
 }  // namespace PEARL_GEOM_NS

@@ -20,8 +20,8 @@
 // per SM; 16: 32x32 tiles, one 512-thread block per SM), into namespaces g8
 // and g16; once more each with the general division, for parameters whose constants
 // the two-operation one is not proved for (g8_div, g16_div); and without the
-// staging, for domains with few tiles a block (plain, plain_wide).  The two cells of a
-// thread share their vertical neighbour loads.
+// staging, for domains with few tiles a block (plain, plain_wide, plain_held).  The
+// two cells of a thread share their vertical neighbour loads.
 // Each phase's input fields are staged per tile by 2-D TMA copies into shared
 // memory through an mbarrier pipeline (`sweep`), which passes over tiles that
 // are uniform; the plain kernels read them from global memory.
@@ -76,6 +76,7 @@ struct Pair {
     size_t i0, i1;                 // centres
     size_t iw0, ie0, iw1, ie1;     // x neighbours (periodic)
     size_t is0, in1;               // y neighbours outside the pair (zero-flux ghost = the cell itself)
+    int pos;                       // position of the tile among the block's (unstaged sweeps only)
 };
 
 __device__ __forceinline__ Pair pair_of(const DevParams& P, int t) {
@@ -336,8 +337,30 @@ __device__ __forceinline__ void list_tiles(Tiles& T, int nb, Take&& take) {
     if (threadIdx.x == 0) T.ndense = n;
 }
 
+// The conjugate-gradient values of a block's cells between the passes of one
+// solve, in shared memory: a slot is written and read by one thread only.  UPDATE
+// then loads nothing from global memory (or p alone, see held_fields) and r, Ap
+// and diag are never stored there; x, z and p still are, for the neighbours and
+// FINAL.  The passes of these domains run from L2 at a few tiles a block, where
+// five planes to load before the first sum are a third of UPDATE's time: 512x1024
+// UPDATE 6.4 -> 5.0 us, SETUP 9.9 -> 8.2, a step 0.1324 -> 0.1213 ms (768x1024
+// 0.1815 -> 0.1735, 512x512 0.0841 -> 0.0786).  The shared memory is L1 that APPLY
+// loses: 6.6 -> 6.6 us at 4 tiles a block, 8.4 -> 9.0 at 6.  A kernel of its own
+// (plain_held), for blocks of 2 to kHeldTiles tiles: beside the other solves in
+// one kernel it cost 380 B of spills, every other pass 0.5-2 us, and one tile a
+// block (diffusion_resident) 0.0566 -> 0.0744 ms a step.
+enum HeldField : int { kHeldX, kHeldR, kHeldAp, kHeldDiag, kHeldP };
+struct Held {
+    double* base = nullptr;
+    int fields = 0;
+    __device__ __forceinline__ double& at(int field, const Pair& c, int cell) const {
+        return base[((c.pos * fields + field) * 2 + cell) * kThreads + threadIdx.x];
+    }
+};
+
 struct Red {
     const Dom& a;
+    Held held;
     Tiles* tiles = nullptr;  // shared memory
     PhaseClock* clk;  // shared memory; used by one thread of block 0 only (keeps_clock)
     unsigned long long counter;  // grid reductions of this block group since the launch began
@@ -583,8 +606,9 @@ __device__ __forceinline__ bool sweep(const Dom& a, Red& red, const int (&maps)[
     const auto tile_of = [&](int k) { return a.bid + (reverse ? nb - 1 - k : k) * G; };
     if (kPlain || !a.use_tma) {
         for (int k = 0; k < nb; ++k) {
-            const Pair c = pair_of(P, tile_of(k));
+            Pair c = pair_of(P, tile_of(k));
             if (!c.v0) continue;
+            c.pos = reverse ? nb - 1 - k : k;
             GlobalSrc<NF, T> src;
 #pragma unroll
             for (int f = 0; f < NF; ++f) src.f[f] = planes[f];
@@ -1113,7 +1137,8 @@ __device__ bool phase_mix(const Dom& a, Red& red, int cur, bool& mixbad) {
 // Slots: K, mu (stencils), chi, icpt, c.  Reduction: {<rhs,rhs>, <r,z>, <r,r>}.
 // kSolve32: the mixed form's set-up (FP32 copies for the inner solve); the FP64
 // kernel is compiled without it.
-template <bool kSolve32>
+// kHeld: r and diag (and x) go to shared memory (Held).
+template <bool kSolve32, bool kHeld>
 __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, double dt, double& rhs2, double& rz, double& rr) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
@@ -1182,7 +1207,8 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
         // the cell's set-up values; the mixed solve keeps the residual and the
         // Jacobi step in FP32 (FP32 copies of the solve's coefficients too) and
         // sums <r,z> of those, <r,r> of the FP64 residual
-        const auto store = [&](size_t i, double chi, const Faces& f, double u0, double rhs, double r, double diag) {
+        const auto store = [&](int cell, double chi, const Faces& f, double u0, double rhs, double r, double diag) {
+            const size_t i = cell ? c.i1 : c.i0;
             B.wE[i] = f.w1;
             B.wN[i] = f.w3;
             B.x[i] = u0;
@@ -1197,9 +1223,15 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
                 s1 += (double)r32 * (double)z32;
             } else {
                 const double z = r / diag;
-                B.r[i] = r;
+                if constexpr (kHeld) {
+                    red.held.at(kHeldX, c, cell) = u0;
+                    red.held.at(kHeldR, c, cell) = r;
+                    red.held.at(kHeldDiag, c, cell) = diag;
+                } else {
+                    B.r[i] = r;
+                    B.diag[i] = diag;
+                }
                 B.z[i] = z;
-                B.diag[i] = diag;
                 s1 += r * z;
             }
             s0 += rhs * rhs;
@@ -1211,7 +1243,7 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
             const double Au = apply0(chi, dt, f, u);
             const double diag = chi + dt * (f.w0 + f.w1 + f.w2 + f.w3);
             const double rhs = cold - ic;
-            store(c.i0, chi, f, u.c0, rhs, rhs - Au, diag);
+            store(0, chi, f, u.c0, rhs, rhs - Au, diag);
         }
         if (c.v1) {
             const double chi = src.v(2, 1, kC), ic = src.v(3, 1, kC), cold = src.v(4, 1, kC);
@@ -1219,7 +1251,7 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
             const double Au = apply1(chi, dt, f, u);
             const double diag = chi + dt * (f.w0 + f.w1 + f.w2 + f.w3);
             const double rhs = cold - ic;
-            store(c.i1, chi, f, u.c1, rhs, rhs - Au, diag);
+            store(1, chi, f, u.c1, rhs, rhs - Au, diag);
         }
     }, uni);
     if (!ok) return false;
@@ -1233,10 +1265,21 @@ __device__ __forceinline__ bool phase_setup(const Dom& a, Red& red, int cur, dou
 
 // APPLY: p_new = z (first) or z + beta*p_old, written to p[pout]; Ap; <p,Ap>.
 // Slots: wE, wN, z (stencils), chi, p_old (stencil).
+template <bool kHeld>
 __device__ __forceinline__ bool phase_apply(const Dom& a, Red& red, double dt, bool first, double beta, int pout, double& pAp) {
     const DevBufs& B = a.B;
     double* pn = B.p[pout];
     double s = 0;
+    const auto store = [&](const Pair& c, int cell, double p, double Ap) {
+        pn[cell ? c.i1 : c.i0] = p;
+        if constexpr (kHeld) {
+            red.held.at(kHeldAp, c, cell) = Ap;
+            if (red.held.fields > kHeldP) red.held.at(kHeldP, c, cell) = p;
+        } else {
+            B.Ap[cell ? c.i1 : c.i0] = Ap;
+        }
+        s += p * Ap;
+    };
     const auto body = [&](const auto& src, const Pair& c) {
         S2 p = stencil2(src, 2, c.v1);
         if (!first) {
@@ -1251,14 +1294,10 @@ __device__ __forceinline__ bool phase_apply(const Dom& a, Red& red, double dt, b
             p.n1 = p.n1 + beta * po.n1;
         }
         const double Ap0 = apply0(src.v(3, 0, kC), dt, faces_stored(src, 0, 1, 0, c), p);
-        pn[c.i0] = p.c0;
-        B.Ap[c.i0] = Ap0;
-        s += p.c0 * Ap0;
+        store(c, 0, p.c0, Ap0);
         if (c.v1) {
             const double Ap1 = apply1(src.v(3, 1, kC), dt, faces_stored(src, 0, 1, 1, c), p);
-            pn[c.i1] = p.c1;
-            B.Ap[c.i1] = Ap1;
-            s += p.c1 * Ap1;
+            store(c, 1, p.c1, Ap1);
         }
     };
     Uniform& U = red.tiles->u;
@@ -1300,6 +1339,7 @@ __device__ __forceinline__ bool phase_apply(const Dom& a, Red& red, double dt, b
 
 // UPDATE: x += alpha p; r -= alpha Ap; z = r/diag; {<r,z>, <r,r>}.
 // Slots (no stencils): x, p, r, Ap, diag.
+template <bool kHeld>
 __device__ __forceinline__ bool phase_update(const Dom& a, Red& red, double alpha, int pcur, double& rz, double& rr) {
     const DevBufs& B = a.B;
     double s0 = 0, s1 = 0;
@@ -1331,24 +1371,31 @@ __device__ __forceinline__ bool phase_update(const Dom& a, Red& red, double alph
             B.z[c.i0] = B.z[c.i1] = U.z;
         });
     const bool ok = sweep<5, true>(a, red, maps, planes, 0x0u, false, [&](const auto& src, const Pair& c) {
-        {
-            const double x = src.v(0, 0, kC) + alpha * src.v(1, 0, kC), r = src.v(2, 0, kC) - alpha * src.v(3, 0, kC);
-            const double z = r / src.v(4, 0, kC);
-            B.x[c.i0] = x;
-            B.r[c.i0] = r;
-            B.z[c.i0] = z;
-            s0 += r * z;
-            s1 += r * r;
-        }
-        if (c.v1) {
-            const double x = src.v(0, 1, kC) + alpha * src.v(1, 1, kC), r = src.v(2, 1, kC) - alpha * src.v(3, 1, kC);
-            const double z = r / src.v(4, 1, kC);
-            B.x[c.i1] = x;
-            B.r[c.i1] = r;
-            B.z[c.i1] = z;
-            s0 += r * z;
-            s1 += r * r;
-        }
+        const auto cell = [&](int k) {
+            const size_t i = k ? c.i1 : c.i0;
+            if constexpr (kHeld) {
+                const double p = red.held.fields > kHeldP ? red.held.at(kHeldP, c, k) : src.v(1, k, kC);
+                const double x = red.held.at(kHeldX, c, k) + alpha * p;
+                const double r = red.held.at(kHeldR, c, k) - alpha * red.held.at(kHeldAp, c, k);
+                const double z = r / red.held.at(kHeldDiag, c, k);
+                red.held.at(kHeldX, c, k) = x;
+                red.held.at(kHeldR, c, k) = r;
+                B.x[i] = x;
+                B.z[i] = z;
+                s0 += r * z;
+                s1 += r * r;
+            } else {
+                const double x = src.v(0, k, kC) + alpha * src.v(1, k, kC), r = src.v(2, k, kC) - alpha * src.v(3, k, kC);
+                const double z = r / src.v(4, k, kC);
+                B.x[i] = x;
+                B.r[i] = r;
+                B.z[i] = z;
+                s0 += r * z;
+                s1 += r * r;
+            }
+        };
+        cell(0);
+        if (c.v1) cell(1);
     }, uni);
     if (!ok) return false;
     double v[2] = {s0, s1};
@@ -1359,6 +1406,7 @@ __device__ __forceinline__ bool phase_update(const Dom& a, Red& red, double alph
 }
 
 // RESET: z = r/diag; <r,z>  (pearl_serial.cpp:1060-1064)
+template <bool kHeld>
 __device__ __forceinline__ bool phase_reset(const Dom& a, Red& red, double& rz) {
     const DevParams& P = a.P;
     const DevBufs& B = a.B;
@@ -1371,14 +1419,20 @@ __device__ __forceinline__ bool phase_reset(const Dom& a, Red& red, double& rz) 
     }
     int pos = 0;
     FOR_TILES(P) {
-        const Pair c = pair_of(P, t);
+        Pair c = pair_of(P, t);
         const int cls = skip ? T.cls[pos] & kClassMask : kDense;
-        ++pos;
+        c.pos = pos++;
         for (int k = 0; k < 2; ++k) {
             if (!(k ? c.v1 : c.v0)) continue;
             const size_t i = k ? c.i1 : c.i0;
             const double r = cls == kDense ? B.r[i] : T.u.r;
-            const double z = cls == kDense ? r / B.diag[i] : T.u.z;
+            double z;
+            if constexpr (kHeld) {  // (the residual that this thread's FINAL wrote)
+                red.held.at(kHeldR, c, k) = r;
+                z = r / red.held.at(kHeldDiag, c, k);
+            } else {
+                z = cls == kDense ? r / B.diag[i] : T.u.z;
+            }
             if (cls != kUniform) B.z[i] = z;
             s += r * z;
         }
@@ -1935,7 +1989,7 @@ constexpr int kMixedMaxRounds = 16;  // FP32 rounds of one mixed solve before th
 __device__ __forceinline__ bool diffusion_mixed(const Dom& a, Red& red, int cur, double dt, DiffusionOut& o) {
     const DevParams& P = a.P;
     double rhs2, rz, rr;
-    if (!phase_setup<true>(a, red, cur, dt, rhs2, rz, rr)) return false;
+    if (!phase_setup<true, false>(a, red, cur, dt, rhs2, rz, rr)) return false;
     const double tolerance = P.cg_atol + P.cg_rtol * sqrt(rhs2);
     double target = fmax(sqrt(rr) * P.inner_rtol, 0.5 * tolerance);  // this round's stop
     bool first = true;
@@ -2181,7 +2235,7 @@ __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, doubl
         if (P.ntiles <= a.nblk) return diffusion_resident(a, red, cur, dt, o);
     }
     double rhs2, rz, rr;
-    if (!phase_setup<false>(a, red, cur, dt, rhs2, rz, rr)) return false;
+    if (!phase_setup<false, kHeldSolve>(a, red, cur, dt, rhs2, rz, rr)) return false;
     const double tolerance = P.cg_atol + P.cg_rtol * sqrt(rhs2);
     bool first = true;
     double beta = 0;
@@ -2202,7 +2256,7 @@ __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, doubl
             o.bad = false;
             o.mass = 0;
             o.energy = 0;
-            if (!phase_reset(a, red, rz)) return false;
+            if (!phase_reset<kHeldSolve>(a, red, rz)) return false;
             first = true;
             continue;
         }
@@ -2212,12 +2266,12 @@ __device__ __forceinline__ bool diffusion(const Dom& a, Red& red, int cur, doubl
         if (!kPlain && red.tiles->active && iteration + 1 >= kReach && !phase_expand<false>(a, red, pbuf)) return false;
         const int pout = pbuf ^ 1;
         double pAp;
-        if (!phase_apply(a, red, dt, first, beta, pout, pAp)) return false;
+        if (!phase_apply<kHeldSolve>(a, red, dt, first, beta, pout, pAp)) return false;
         pbuf = pout;
         if (!(pAp > 0) || !isfinite(pAp) || !isfinite(rz)) return true;
         const double alpha = rz / pAp;
         double rz_next;
-        if (!phase_update(a, red, alpha, pbuf, rz_next, rr)) return false;
+        if (!phase_update<kHeldSolve>(a, red, alpha, pbuf, rz_next, rr)) return false;
         beta = rz_next / rz;
         rz = rz_next;
         first = false;
@@ -2822,6 +2876,10 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
     Red red(a, &clk);
     red.pipe_ptr = &pipe;
     red.tiles = &tiles;
+    if (kHeldSolve) {
+        red.held.base = reinterpret_cast<double*>(dsmem);
+        red.held.fields = args.held_fields;
+    }
     StepState st;
     st.S = ctl->S;
     st.cur = ctl->cur;
@@ -2843,7 +2901,7 @@ __device__ __forceinline__ void step_body(const KArgs& args) {
             }
             pearl_step_info info;
             if (args.forced_dt) st.S.dt = args.forced_dt[steps];
-            if (!advance<kSolve32, kPlain>(a, red, st, args.L.stop_time, info)) break;
+            if (!advance<kSolve32, kPlain && !kHeldSolve>(a, red, st, args.L.stop_time, info)) break;
             if (args.dt_log && leader) args.dt_log[steps] = info.accepted_dt;
             if (args.hist && leader) args.hist[(args.hist_next + steps) % args.hist_cap] = info;
             if (args.tape) record_tape(a, st.cur, args.tape + args.tape_slot * steps);

@@ -68,8 +68,9 @@ void set_tile_shape(pearl_gpu_ctx* ctx, int wx_log2);
 enum StepKernel { kStepRun, kStepRunMixed, kStepModes };
 const void* step_kernel(int warps, StepKernel kind, bool fast_div);
 // The step loop of a domain of 8-warp blocks that does not stage: compiled for
-// one block per SM where the grid allows that, else for two.
-const void* plain_step_kernel(int grid, int sms);
+// one block per SM where the grid allows that, else for two; held: the one for
+// KArgs::held_fields > 0.
+const void* plain_step_kernel(int grid, int sms, bool held);
 // Shared memory opt-in of a kernel, and the check that `grid` blocks of it are co-resident.
 cudaError_t prepare_kernel(const void* kernel, int threads, size_t smem, int grid, int sms);
 // pearl_gpu_create; prepare: with the step kernel of a context of its own (an

@@ -51,7 +51,24 @@ struct KArgs {
     long long hist_cap, hist_next;
     // run mode: leave the state in set 0 (the no-allocation step's caller planes)
     int end_in_set0;
+    // run mode of plain_held: fields of a cell that the solve keeps in (dynamic)
+    // shared memory, held_bytes of it
+    int held_fields;
 };
+
+// The solve's values of a cell in plain_held (Held): 4 KB a field and tile.  Two
+// blocks an SM leave 113 KB a block: all five fields up to 5 tiles, four (UPDATE
+// reads p from its plane) at 6, the most tiles a block has below the staging rule.
+// One tile a block is held in registers.
+constexpr int kHeldTiles = 6;
+constexpr int held_fields(long long tiles, long long grid) {
+    const long long most = (tiles + grid - 1) / grid;
+    return most < 2 || most > kHeldTiles ? 0 : most == kHeldTiles ? 4 : 5;
+}
+constexpr size_t kHeldMaxBytes = 5 * (kHeldTiles - 1) * 512 * sizeof(double);
+constexpr size_t held_bytes(long long tiles, long long grid, int threads) {
+    return (size_t)held_fields(tiles, grid) * (size_t)((tiles + grid - 1) / grid) * 2 * threads * sizeof(double);
+}
 
 // One instance of a batch: its tensor maps, parameters and buffers.
 struct alignas(64) BatchInstance {
@@ -128,12 +145,16 @@ PEARL_DECLARE_KERNELS(8, 2)
 namespace g16_div {
 PEARL_DECLARE_KERNELS(16, 1)
 }
-// The step loop of one domain that does not stage: two blocks per SM, and one.
+// The step loop of one domain that does not stage: two blocks per SM, one, and two
+// that keep the solve's values in shared memory.
 namespace plain {
 __global__ void __launch_bounds__(256, 2) pearl_kernel(const __grid_constant__ KArgs args);
 }
 namespace plain_wide {
 __global__ void __launch_bounds__(256, 1) pearl_kernel(const __grid_constant__ KArgs args);
+}
+namespace plain_held {
+__global__ void __launch_bounds__(256, 2) pearl_kernel(const __grid_constant__ KArgs args);
 }
 #undef PEARL_DECLARE_KERNELS
 static_assert(tile_geometry(8).min_blocks == 2 && tile_geometry(16).min_blocks == 1, "kernel launch bounds");

@@ -134,7 +134,7 @@ extern "C" int pearl_gpu_advance_noalloc(const pearl_params* params, int nx, int
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return PEARL_ERR_CUDA;
     const void* const kernel =
-        ctx.P.fast_div ? plain_step_kernel(ctx.P.ntiles, sms) : step_kernel(8, kStepRun, false);
+        ctx.P.fast_div ? plain_step_kernel(ctx.P.ntiles, sms, false) : step_kernel(8, kStepRun, false);
     // the blocks per SM that the kernels are compiled for; a device that cannot hold
     // them refuses the cooperative launch
     const int grid =

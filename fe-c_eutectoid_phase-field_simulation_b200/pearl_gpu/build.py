@@ -31,8 +31,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_SOURCES = [
     *((f"pearl_fp64_g{w}" + ("" if fast else "_div"), "pearl_fp64.cu",
        ["-fmad=false", f"-DPEARL_TILE_WARPS={w}", f"-DPEARL_FAST_DIV={fast}"]) for w in (8, 16) for fast in (1, 0)),
-    # the step loop of domains that do not stage: two blocks per SM, and one
-    *((f"pearl_fp64_plain{n}", "pearl_fp64.cu", ["-fmad=false", f"-DPEARL_PLAIN={n}"]) for n in (1, 2)),
+    # the step loop of domains that do not stage: two blocks per SM, one, and two
+    # that keep the solve's values in shared memory
+    *((f"pearl_fp64_plain{n}", "pearl_fp64.cu", ["-fmad=false", f"-DPEARL_PLAIN={n}"]) for n in (1, 2, 3)),
     ("pearl_ctx", "pearl_ctx.cu", ["-fmad=false"]),            # context, transfers, single-domain C ABI
     ("pearl_batch", "pearl_batch.cu", ["-fmad=false"]),        # batched instances
     ("pearl_adjoint_host", "pearl_adjoint_host.cu", ["-fmad=false"]),  # adjoint gradient driver
