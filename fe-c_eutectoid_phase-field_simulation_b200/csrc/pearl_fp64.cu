@@ -45,6 +45,7 @@
 #include <cudaTypedefs.h>
 
 #include "pearl_kernels.cuh"
+#include "pearl_uniform.hpp"
 
 namespace pearl_gpu {
 namespace PEARL_GEOM_NS {  // compiled once per block shape (PEARL_TILE_WARPS = 8, 16)
@@ -292,7 +293,7 @@ struct Uniform {
     double ref[5];            // the reference cell: phi (3), mu, carbon
     double q0, q1, q2, change;  // its proposal
     double K, chi, icpt;
-    int have, simplex_bad, mix_bad;
+    int simplex_bad, mix_bad;
     Faces f;
     double x, r, z, p, Ap, diag, cn, mun, closure;
     bool held;  // the trial set already holds (mun, cn) in every uniform tile
@@ -881,7 +882,8 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
     Uniform& U = T.u;
     const int set = cur ^ 1, nb = a.bid < P.ntiles ? (P.ntiles - 1 - a.bid) / a.nblk + 1 : 0;
     bool skipping = false;  // the far tiles are known to be uniform
-    bool same = true, have = false;  // this thread's cells of the tile are uniform; U holds their proposal
+    bool same = true;    // this thread's cells of the tile are uniform
+    FilledByVote first;  // U holds their proposal
     if constexpr (kFindUniform) {
         maps[4] = kMapState + 5 * cur + 3;
         planes[4] = B.c[cur];
@@ -889,10 +891,7 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
             // reference cell: some rows below the top wall, where the austenite has been longest
             const size_t i = (size_t)(P.ny - 1 - P.ny / 16) * P.pitch + P.nx / 2;
             if (threadIdx.x < 5) U.ref[threadIdx.x] = planes[threadIdx.x][i];
-            if (threadIdx.x == 0) {
-                U.have = 0;
-                T.active = 0;
-            }
+            if (threadIdx.x == 0) T.active = 0;
             __syncthreads();
             skipping = T.known;
 #pragma unroll
@@ -932,7 +931,7 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
     const auto body = [&](auto mixed_tag, const auto& src, const Pair& c) {
         if (find) {
             same = equals_ref(src, c);
-            if (same && have) {
+            if (first.takes(same)) {
                 vchange = fmax(vchange, U.change);
                 if (U.simplex_bad) vsimp = 1;
                 if (U.mix_bad) vmix = 1;
@@ -976,7 +975,7 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
                 B.c[cur ^ 1][i] = fma(chi, mu, cint);
                 B.mu[cur ^ 1][i] = mu;
             }
-            if (kFindUniform && find && same && k == 0 && threadIdx.x == 0) {
+            if (kFindUniform && find && k == 0 && first.fills(same, threadIdx.x == 0)) {
                 U.q0 = o.z0;
                 U.q1 = o.z1;
                 U.q2 = o.z2;
@@ -986,7 +985,6 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
                 U.K = K;
                 U.chi = chi;
                 U.icpt = icpt;
-                U.have = 1;
             }
         }
     };
@@ -1002,7 +1000,7 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
             h = (unsigned char)((h & ~(1 << set)) | (all << set));
         }
         same = true;  // lanes outside the domain have no say
-        if (!have) have = U.have != 0;
+        first.vote(all);
     };
     using Uni = std::conditional_t<kFindUniform, ReadListed, NoUniform>;
     const bool ok =
