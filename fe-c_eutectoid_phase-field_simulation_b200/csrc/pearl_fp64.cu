@@ -461,6 +461,12 @@ struct SmemSrc {
     }
 };
 
+// A cell whose neighbours all equal it.
+struct RefSrc {
+    const double* ref;
+    __device__ __forceinline__ double v(int k, int, int) const { return ref[k]; }
+};
+
 // Both cells' five-point stencils of slot k (see S2); the upper cell's own
 // neighbours are only read when it is inside the domain.
 template <class Src>
@@ -866,7 +872,12 @@ __device__ __forceinline__ Proposal propose_cell_mixed(const DevParams& P, const
 // beside phi and mu for that, 8 bytes a cell in a phase that its arithmetic
 // bounds.  A cell that equals the reference cell with its neighbours takes the
 // proposal computed at the first such cell of the block.
-template <bool kFindUniform>
+// kEveryBlock: a block without a uniform tile forms that proposal too, from the
+// reference cell.  The mixed solve needs it: UPDATE32 walks the whole domain, where
+// the other passes add a uniform tile's value in the tile's own block.  (One
+// thread's 4 us a step: 1024x1024 with its front at 0.85 0.284 -> 0.288 ms; nothing
+// where every block has a uniform tile, 2048x4096 in its window 0.929.)
+template <bool kFindUniform, bool kEveryBlock = false>
 __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, double dt, double& change, bool& mixbad,
                               bool& simplexbad) {
     const DevParams& P = a.P;
@@ -926,6 +937,17 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
         }
         return d == 0;
     };
+    const auto leave = [&](const Proposal& o, bool mix, double K, double chi, double icpt) {
+        U.q0 = o.z0;
+        U.q1 = o.z1;
+        U.q2 = o.z2;
+        U.change = o.change;
+        U.simplex_bad = o.simplex_bad;
+        U.mix_bad = !mix;
+        U.K = K;
+        U.chi = chi;
+        U.icpt = icpt;
+    };
     // the FP64 and the mixed-precision proposal are separate sweeps, so each
     // loop is register-allocated on its own
     const auto body = [&](auto mixed_tag, const auto& src, const Pair& c) {
@@ -975,17 +997,7 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
                 B.c[cur ^ 1][i] = fma(chi, mu, cint);
                 B.mu[cur ^ 1][i] = mu;
             }
-            if (kFindUniform && find && k == 0 && first.fills(same, threadIdx.x == 0)) {
-                U.q0 = o.z0;
-                U.q1 = o.z1;
-                U.q2 = o.z2;
-                U.change = o.change;
-                U.simplex_bad = o.simplex_bad;
-                U.mix_bad = !mix;
-                U.K = K;
-                U.chi = chi;
-                U.icpt = icpt;
-            }
+            if (kFindUniform && find && k == 0 && first.fills(same, threadIdx.x == 0)) leave(o, mix, K, chi, icpt);
         }
     };
     const auto tile_end = [&](int t) {
@@ -1010,6 +1022,14 @@ __device__ __forceinline__ bool phase_propose(const Dom& a, Red& red, int cur, d
                             [&](const auto& src, const Pair& c) { body(std::false_type{}, src, c); }, Uni{}, tile_end);
     if (!ok) return false;
     if (find) {
+        if (kEveryBlock && !first.filled && threadIdx.x == 0) {
+            const RefSrc src{U.ref};
+            const Proposal o =
+                P.mixed ? propose_cell_mixed(P, src, 0, dt, true, true) : propose_cell(P, src, 0, dt, true, true);
+            double chi, cint, K;
+            const bool mix = mixture(P, o.z0, o.z1, o.z2, chi, cint, K);
+            leave(o, mix, K, chi, fma(chi, P.mu_ref, cint));
+        }
         __syncthreads();
         if (skipping) {
             // the tiles left out: their proposal is U's; written where the trial set holds another
@@ -2318,7 +2338,8 @@ __device__ __forceinline__ bool advance(const Dom& a, Red& red, StepState& st, d
         out.retries = attempt;
         out.accepted_dt = dt;
         bool mixbad, simplexbad;
-        if (!phase_propose<!kPlain>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad)) return false;
+        if (!phase_propose<!kPlain, kSolve32>(a, red, st.cur, dt, out.max_phase_change, mixbad, simplexbad))
+            return false;
         if (simplexbad) {
             set_error(a, PEARL_ERR_SIMPLEX, 0);
             return false;
