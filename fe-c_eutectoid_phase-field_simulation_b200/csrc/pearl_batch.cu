@@ -33,6 +33,7 @@ struct pearl_gpu_batch {
     std::vector<double> dense;        // estimated dense tiles of each instance's uploaded state (0: not known)
     bool replan = false;              // states uploaded since the groups were last sized
     std::vector<int> sizes;           // blocks of each group
+    std::vector<std::vector<int>> lists;  // its instances
     const void* prepared = nullptr;  // kernel of the last launch, and its staging
     bool prepared_tma = false;
     double pass_overhead_tiles = 4;  // sized groups: fixed cost of a pass, in tiles of one block
@@ -233,6 +234,7 @@ int batch_set_groups(pearl_gpu_batch* b, const std::vector<int>& sizes, const st
     b->ngroups = (int)sizes.size();
     b->grid = (int)block_group.size();
     b->sizes = sizes;
+    b->lists = lists;
     return PEARL_OK;
 }
 
@@ -258,7 +260,7 @@ int batch_replan(pearl_gpu_batch* b) {
     const std::vector<int> sizes = groups_by_work(b->dense, tiles, max_grid);
     std::vector<std::vector<int>> lists(b->n);
     for (int i = 0; i < b->n; ++i) lists[i] = {i};
-    if (sizes == b->sizes) return PEARL_OK;
+    if (sizes == b->sizes && lists == b->lists) return PEARL_OK;
     PB_CUDA(b, cudaSetDevice(b->device));
     return batch_set_groups(b, sizes, lists);
 }
