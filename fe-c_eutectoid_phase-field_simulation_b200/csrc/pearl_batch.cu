@@ -31,7 +31,8 @@ struct pearl_gpu_batch {
     double* d_group_part = nullptr;
     int per_sm = 0, sms = 0, grid = 0, group_blocks = 0, ngroups = 0;  // group_blocks -1: sized per instance
     std::vector<double> dense;        // estimated dense tiles of each instance's uploaded state (0: not known)
-    bool replan = false;              // states uploaded since the groups were last sized
+    std::vector<char> fresh;          // instances uploaded since the last run
+    bool replan = false;              // sized groups are due to be sized by the uploaded states
     std::vector<int> sizes;           // blocks of each group
     std::vector<std::vector<int>> lists;  // its instances
     const void* prepared = nullptr;  // kernel of the last launch, and its staging
@@ -238,10 +239,12 @@ int batch_set_groups(pearl_gpu_batch* b, const std::vector<int>& sizes, const st
     return PEARL_OK;
 }
 
-// Groups sized per instance follow the states uploaded since they were last
-// sized: the tiles that an instance's passes leave out (uniform austenite) cost
-// next to nothing, and one instance with its front high up would otherwise hold
-// the launch.  Only where the grid has two blocks an instance and fewer than its
+// Groups sized per instance follow the uploaded states: the tiles that an
+// instance's passes leave out (uniform austenite) cost next to nothing, and one
+// instance with its front high up would otherwise hold the launch.  A group's size
+// is the order of its instances' sums, so the groups are sized again only for a
+// new sweep (all instances uploaded since the last run) or a new configuration: a
+// new state for some of them leaves the others their bits.  Only where the grid has two blocks an instance and fewer than its
 // tiles: below that, groups run several instances and plan_groups balances them;
 // above, every tile has a block.  96 instances of 32..192 x 64..1024 cells, 20
 // steps: 25.7 -> 19.7 ms; 24 instances 7.7 -> 5.2.
@@ -399,6 +402,7 @@ int pearl_gpu_batch_create(int n, const pearl_params* params, const int* nx, con
     if (cudaSetDevice(device) != cudaSuccess) return bail(PEARL_ERR_NO_DEVICE);
     b->inst.assign(n, nullptr);
     b->dense.assign(n, 0.0);
+    b->fresh.assign(n, 0);
     if (cudaMalloc(&b->d_ctls, sizeof(Ctl) * n) != cudaSuccess ||
         cudaMallocHost(&b->h_ctls, sizeof(Ctl) * n) != cudaSuccess ||
         cudaMalloc(&b->d_inst, sizeof(BatchInstance) * n) != cudaSuccess)
@@ -439,7 +443,8 @@ int pearl_gpu_batch_upload(pearl_gpu_batch* b, int i, const double* phi, const d
     const int rc = pearl_gpu_upload(b->inst[i], phi, carbon, mu, scalars);
     if (rc) return bfail(b, rc, pearl_gpu_last_error(b->inst[i]));
     b->dense[i] = phi && carbon && mu ? dense_tiles(b->inst[i], phi, carbon, mu) : 0;
-    b->replan = true;
+    b->fresh[i] = 1;
+    if (std::find(b->fresh.begin(), b->fresh.end(), 0) == b->fresh.end()) b->replan = true;
     return PEARL_OK;
 }
 
@@ -458,6 +463,7 @@ int pearl_gpu_batch_run(pearl_gpu_batch* b, const pearl_run_limits* limits, pear
     if (rc) return rc;
     rc = batch_launch(b, *limits);
     if (rc) return rc;
+    std::fill(b->fresh.begin(), b->fresh.end(), 0);
     int first_bad = PEARL_OK;
     for (int i = 0; i < b->n; ++i) {
         const Ctl& h = b->h_ctls[i];

@@ -377,8 +377,15 @@ int pearl_gpu_adjoint_gradient(pearl_gpu_ctx* ctx, long long nsteps, int checkpo
  * finishes soonest under a model of a pass's cost (powers of two up to the
  * grid, or an equal share of the grid per instance): small instances share
  * groups of a few blocks, large ones get many.  With two blocks or more
- * an instance, the sizes follow the uploaded states: an instance gets blocks in
- * proportion to the part of it that is not uniform austenite.  Every instance follows exactly the path of a
+ * an instance, and fewer than one a tile, the sizes follow the uploaded states:
+ * an instance gets blocks in proportion to the part of it that is not uniform
+ * austenite.  They are set at the first run after all instances have been
+ * uploaded with no run between, or (all of them uploaded before) after the batch
+ * was configured, and kept through other runs and uploads.  The order of an instance's sums, and with it the last bits
+ * of its results, depends on its group's size, here on all the states uploaded
+ * for a sweep: a sweep that is downloaded and uploaded again half-way agrees with the
+ * uninterrupted one to rounding.  Groups of one given size (group_blocks > 0)
+ * repeat it bit for bit.  Every instance follows exactly the path of a
  * pearl_gpu_ctx (same kernels, same reduction order for the same group size),
  * so it is main's loop (pearl_serial.cpp:2296-2306) run once per instance.
  * No counterpart in the reference, which runs one case per process. */
