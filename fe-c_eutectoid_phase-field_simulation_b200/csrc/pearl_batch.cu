@@ -506,7 +506,8 @@ int pearl_gpu_batch_autotune(pearl_gpu_batch* b, int steps, int* group_blocks, i
     bool best_tma = b->use_tma;
     double best_o = b->pass_overhead_tiles;
     // equal groups of 1..16 blocks, and groups sized per instance with three
-    // weights of a pass's fixed cost (in tiles of one block)
+    // weights of a pass's fixed cost (in tiles of one block; where the uploaded
+    // states size the groups they do so whatever the weight)
     struct Cand {
         int gb;
         double o;
@@ -533,6 +534,7 @@ int pearl_gpu_batch_autotune(pearl_gpu_batch* b, int steps, int* group_blocks, i
             if (gb > b->per_sm * b->sms) continue;
             if (gb == PEARL_BATCH_SIZED_GROUPS) b->pass_overhead_tiles = cand.o;
             int rc = batch_configure(b, gb, tma != 0, sh.wx);
+            if (rc == PEARL_OK) rc = batch_replan(b);  // the groups that a run would use
             double ms = 0;
             if (rc == PEARL_OK) {
                 rc = batch_launch(b, L);
@@ -563,7 +565,8 @@ int pearl_gpu_batch_autotune(pearl_gpu_batch* b, int steps, int* group_blocks, i
     }
     release();
     b->pass_overhead_tiles = best_o;
-    const int rc = batch_configure(b, best_gb, best_tma, best_wx);
+    int rc = batch_configure(b, best_gb, best_tma, best_wx);
+    if (rc == PEARL_OK) rc = batch_replan(b);
     if (group_blocks) *group_blocks = best_gb;
     if (use_tma) *use_tma = best_tma ? 1 : 0;
     if (tile_warps_x) *tile_warps_x = 1 << best_wx;

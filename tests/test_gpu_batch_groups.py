@@ -37,13 +37,10 @@ def _dense(w):
     return -(-nx // 32) * (rows - left_out + 0.05 * left_out)
 
 
-def _tiles():
-    return [-(-nx // 32) * -(-ny // 16) for nx, ny in SIZES]
-
-
 def _groups(ws):
     """The smallest m for which groups of ceil(dense / m) blocks fit the grid."""
-    dense, tiles = [_dense(w) for w in ws], _tiles()
+    dense = [_dense(w) for w in ws]
+    tiles = [-(-w.nx // 32) * -(-w.ny // 16) for w in ws]
 
     def sizes(m):
         return [int(max(1.0, min(float(t), math.ceil(d / m)))) for d, t in zip(dense, tiles)]
@@ -124,3 +121,23 @@ def test_one_new_state_leaves_the_others_their_bits(batch, port):
     reports = _run(batch, 2)
     for i, w in enumerate(ws):
         _check(port, batch, reports, i, w, _groups(ws)[i], 2)
+
+
+def test_autotune_leaves_the_groups_that_run(gpu_lib):
+    """On domains large enough for staging to win, and with most of them uniform."""
+    import pearl_gpu
+    from pearl_gpu import workloads
+
+    ws = [workloads.scaled(nx, ny, seed=k, undercooling=20.0, dt=4e-12, dt_max=8e-12, front=front)
+          for k, (nx, ny, front) in enumerate([(640, 1500, 60.0), (512, 1200, 500.0), (400, 1600, 200.0)])]
+    tiles = [-(-w.nx // 32) * -(-w.ny // 16) for w in ws]
+    sizes = _groups(ws)
+    _, planned, _ = pearl_gpu.batch_plan(tiles, GRID, pearl_gpu.BATCH_SIZED_GROUPS)
+    assert sum(planned) != sum(sizes)
+    with pearl_gpu.Batch([(w.params, w.nx, w.ny) for w in ws]) as b:
+        _upload(b, ws)
+        # equal groups of up to 16 blocks would leave most of the grid idle
+        assert b.autotune(steps=2) == (pearl_gpu.BATCH_SIZED_GROUPS, True, 1)
+        timed = b.stats()["grid"]
+        _run(b, 2)
+        assert timed == b.stats()["grid"] == sum(sizes)
