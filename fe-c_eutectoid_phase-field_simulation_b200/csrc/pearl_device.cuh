@@ -121,6 +121,21 @@ __device__ __forceinline__ double div_by(const DevParams& P, double a, double b,
     return P.exact_div ? div_corrected(a, b, rb) : a / b;
 }
 
+// div_by without its operand tests, for positive divisors where neither the sign
+// of an infinite quotient nor a choice between Inf and NaN matters: the same
+// quotient for finite numerators and quotients.  A zero numerator's sign is OR-ed
+// into the result (the corrections turn -0 into +0, and a nonzero quotient
+// already has the numerator's sign); a non-finite numerator gives NaN.
+__device__ __forceinline__ double div_force(const DevParams& P, double a, double b, double rb) {
+    if (!P.exact_div) return a / b;
+    const double q0 = a * rb;
+    double r = fma(-q0, b, a);
+    double q = fma(r, rb, q0);
+    r = fma(-q, b, a);
+    q = fma(r, rb, q);
+    return __hiloint2double(__double2hiint(q) | (__double2hiint(a) & (int)0x80000000), __double2loint(q));
+}
+
 namespace PEARL_GEOM_NS {
 // a/b, correctly rounded, for a divisor with constants zh and zl that
 // exact_reciprocal has proved right for every normal numerator: two dependent
@@ -133,11 +148,12 @@ namespace PEARL_GEOM_NS {
 // pearl_serial.cpp:990-996, whatever its value; an energy squares its
 // quotients, and a non-finite trial fails valid_state first.)  The kernels of
 // the general namespaces, for the one parameter set in a hundred with a divisor
-// that exact_reciprocal refuses, divide with div_by: a choice inside one kernel
-// puts a branch at every quotient, which held PROPOSE at 183 us on 2048x4096.
+// that exact_reciprocal refuses, divide with div_force, which asks for no more: a
+// choice inside one kernel puts a branch at every quotient, which held PROPOSE at
+// 183 us on 2048x4096.
 __device__ __forceinline__ double div_const(const DevParams& P, double a, double b, double zh, double zl) {
     if constexpr (PEARL_FAST_DIV != 0) return fma(a, zh, a * zl);
-    return div_by(P, a, b, zh);
+    return div_force(P, a, b, zh);
 }
 }  // namespace PEARL_GEOM_NS
 
