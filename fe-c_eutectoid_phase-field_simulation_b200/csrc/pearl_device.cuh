@@ -138,7 +138,8 @@ __device__ __forceinline__ double div_force(const DevParams& P, double a, double
 
 namespace PEARL_GEOM_NS {
 // a/b, correctly rounded, for a divisor with constants zh and zl that
-// exact_reciprocal has proved right for every normal numerator: two dependent
+// exact_reciprocal has proved right for every quotient of at least 2^-916 (below,
+// a last bit that no result hangs on, pearl_division.hpp): two dependent
 // FP64 operations where div_by takes five and its integer tests (PROPOSE has 20
 // of these divisions a cell, FINAL 10, and both are bound by FP64 issue and
 // latency).  The sign of a zero numerator may be lost and a non-finite

@@ -4,12 +4,21 @@
 // zl close to 1/b - zh, and a/b by RN(a*zh + RN(a*zl)): one multiplication and
 // one fused multiply-add (Brisebarre, Muller, Raina, "Accelerating correctly
 // rounded floating-point division when the divisor is known in advance", IEEE
-// Trans. Comput. 53(8), 2004).  The result is the correctly rounded quotient
-// for every normal a with a normal quotient unless a/b lies closer to the
+// Trans. Comput. 53(8), 2004).  As long as a*zl is a normal number, the result is
+// the correctly rounded quotient unless a/b lies closer to the
 // midpoint of two neighbouring doubles than the method's error, and for one b
 // only a handful of significands a come that close: they solve
 // a 2^s = m b + n with m odd and |n| small.  exact_reciprocal() solves for them
-// and tries each, so a pair that it returns is right for all a.
+// and tries each, so a pair that it returns is right for all a of that range.
+//
+// The range: 1 - b zh is a multiple of 2^-105, so |a*zl| is at least about
+// 2^-105 |a/b| (or zl is 0 and a*zh exact), and every quotient from kExactFrom up
+// to the largest double is in it.  Below, a*zl loses bits to underflow, and a normal
+// quotient may be one unit in the last place off (1 of 300 numerators between
+// 2^-1000 and 2^-980 at b = 9.4e6).  No result hangs on that unit: a force's
+// quotient is added to obstacle terms of some 1e7, a face weight to a
+// susceptibility, a gradient's energy is its square, and what a chemical energy or
+// a phase's composition divides is 0 or a difference of numbers far above that range.
 #pragma once
 
 #include <cmath>
@@ -17,6 +26,9 @@
 #include <initializer_list>
 
 namespace pearl_gpu {
+
+// The smallest |a/b| whose rounding exact_reciprocal answers for.
+constexpr double kExactFrom = 0x1p-916;
 
 namespace division_detail {
 
@@ -59,8 +71,8 @@ bool near_midpoints(uint64_t B, F&& f) {
 
 }  // namespace division_detail
 
-// Constants (zh, zl) for the divisor b, true when they give a/b for all normal
-// a with a normal quotient.  zl is 1/b - zh rounded, or a neighbour of it where
+// Constants (zh, zl) for the divisor b, true when they give a/b for all a with
+// |a/b| from kExactFrom to the largest double.  zl is 1/b - zh rounded, or a neighbour of it where
 // that one misses a quotient (about one divisor in 160); for one divisor in a
 // thousand none of the three does, and the kernels of the general division run.
 inline bool exact_reciprocal(double b, double& zh, double& zl) {
