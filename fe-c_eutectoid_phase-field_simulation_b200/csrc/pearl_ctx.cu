@@ -660,14 +660,21 @@ int pearl_gpu::create_context(const pearl_params* params, int nx, int ny, int de
     if (!coop) return bail(PEARL_ERR_NO_DEVICE);
     // Block shape: 8 warps (two 256-thread blocks per SM, 32x16 tiles) up to 160
     // 32x32 tiles per SM, 16 warps (512 threads, one block per SM, 32x32 tiles)
-    // beyond.  With uniform tiles left out, the finer tiles follow the dense part
-    // of a domain more closely (ms per step, 8 against 16 warps, front at 0.1 and
-    // 0.5 of the height: 1000x1537, 10 tiles per SM, 0.152 against 0.169, at 0.45
-    // 0.250 against 0.266; 2048x4096, 55 tiles, at its start 0.195 against 0.231,
-    // 0.872 against 0.888; 4096x4096, 111 tiles, 0.506 against 0.565, 1.690 against
-    // 1.696); on the largest domains half the blocks in every barrier and 5% fewer
-    // halo bytes count more (4096x8192, 221 tiles, 0.848 against 0.889 at 0.1 but
-    // 3.315 against 3.216 at 0.5).  PEARL_GPU_TILE_WARPS = 8 or 16 overrides.
+    // beyond.  With uniform tiles left out, the finer tiles follow the dense part of a
+    // domain more closely; a domain that is all dense, and the largest ones, gain more
+    // from half the blocks in every barrier and 5% fewer halo bytes.  ms per step, 8
+    // against 16 warps:
+    //                tiles/SM   front at 0.1    at 0.5         no uniform tile
+    //   1000x1537     11        0.162 / 0.186   0.272 / 0.290   0.377 / 0.379
+    //   2048x2048     28        0.256 / 0.285   0.539 / 0.573   0.845 / 0.840
+    //   2048x4096     55        0.352 / 0.385   0.937 / 0.955   1.672 / 1.595
+    //   4096x4096    111        0.605 / 0.666   1.819 / 1.815   3.333 / 3.168
+    //   4096x6144    166        0.822 / 0.881   2.706 / 2.633   5.130 / 4.867
+    //   4096x8192    221        1.022 / 1.070   3.583 / 3.474   6.860 / 6.603
+    // The rule is for fronts in the window's range and below it.  A dense domain of 55
+    // to 160 tiles per SM loses up to 5%, the mixed forms there 6%, and
+    // pearl_gpu_implicit_diffusion, which is always dense, 7%.
+    // PEARL_GPU_TILE_WARPS = 8 or 16 overrides.
     {
         const long long tiles16 = (long long)((nx + 31) / 32) * ((ny + 31) / 32);
         ctx->warps = tiles16 >= 160LL * sms ? 16 : 8;
@@ -685,12 +692,20 @@ int pearl_gpu::create_context(const pearl_params* params, int nx, int ny, int de
     // PEARL_GPU_GRID caps the block count (the grid-size sweeps of small domains)
     if (const char* e = std::getenv("PEARL_GPU_GRID"))
         if (std::atoi(e) > 0) ctx->grid = std::min(ctx->grid, std::atoi(e));
-    // TMA staging pays once a block has a few tiles per pass to pipeline; with
-    // fewer, the pipeline's fill and proxy fences cost more than plain loads
-    // (1965 MHz, one GPU: 768x1024, 5.2 tiles a block, 0.258 staged against
-    // 0.234 ms/step plain; 1024x1024, 6.9 tiles, 0.300 against 0.304;
-    // 1024x2048, 13.8 tiles, 0.497 against 0.601; 256x512 0.0947 against
-    // 0.0733).  PEARL_GPU_TMA=1 stages whatever the size, =0 never.
+    // TMA staging pays once a block has a few tiles per pass to pipeline, and sooner
+    // where uniform tiles are left out, which only the staged kernels do; below, the
+    // pipeline's fill and proxy fences cost more than plain loads, whose kernels keep
+    // the solve's values on the chip.  ms per step, staged against plain:
+    //             tiles a block  front at 0.1    at 0.35         at 0.6          no uniform tile
+    //   512x592       2.0        0.104 / 0.086   0.118 / 0.082   0.117 / 0.079   0.117 / 0.076
+    //   512x1184      4.0        0.105 / 0.130   0.135 / 0.125   0.175 / 0.122   0.187 / 0.116
+    //   512x1480      5.0        0.121 / 0.176   0.166 / 0.169   0.223 / 0.173   0.234 / 0.166
+    //   768x1184      6.0        0.127 / 0.192   0.171 / 0.184   0.218 / 0.180   0.230 / 0.171
+    //   1024x1024     6.9        0.153 / 0.245   0.197 / 0.236   0.234 / 0.232   0.255 / 0.224
+    //   1024x1184     8.0        0.142 / 0.309   0.198 / 0.296   0.244 / 0.290   0.284 / 0.283
+    //   1024x1536    10.4        0.163 / 0.437   0.230 / 0.422   0.296 / 0.436   0.376 / 0.425
+    // Six tiles a block: the lines cross between 4 and 8, by the front's height, which
+    // the rule does not know.  PEARL_GPU_TMA=1 stages whatever the size, =0 never.
     ctx->stage_tma = ctx->use_tma && ((tma_env && std::atoi(tma_env) != 0) || ctx->P.ntiles >= 6LL * ctx->grid);
     if (prepare) {
         cudaError_t e;
