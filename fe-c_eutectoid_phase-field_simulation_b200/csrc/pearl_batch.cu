@@ -31,6 +31,7 @@ struct pearl_gpu_batch {
     double* d_group_part = nullptr;
     int per_sm = 0, sms = 0, grid = 0, group_blocks = 0, ngroups = 0;  // group_blocks -1: sized per instance
     std::vector<double> dense;        // estimated dense tiles of each instance's uploaded state (0: not known)
+    bool by_state = false;            // sized groups follow the uploaded states, not the tile counts alone
     std::vector<char> fresh;          // instances uploaded since the last run
     bool replan = false;              // sized groups are due to be sized by the uploaded states
     std::vector<int> sizes;           // blocks of each group
@@ -239,20 +240,23 @@ int batch_set_groups(pearl_gpu_batch* b, const std::vector<int>& sizes, const st
     return PEARL_OK;
 }
 
-// Groups sized per instance follow the uploaded states: the tiles that an
-// instance's passes leave out (uniform austenite) cost next to nothing, and one
-// instance with its front high up would otherwise hold the launch.  A group's size
-// is the order of its instances' sums, so the groups are sized again only for a
-// new sweep (all instances uploaded since the last run) or a new configuration: a
-// new state for some of them leaves the others their bits.  Only where the grid has two blocks an instance and fewer than its
-// tiles: below that, groups run several instances and plan_groups balances them;
-// above, every tile has a block.  96 instances of 32..192 x 64..1024 cells, 20
-// steps: 25.7 -> 19.7 ms; 24 instances 7.7 -> 5.2.
+// The default's groups follow the uploaded states: the tiles that an instance's
+// passes leave out (uniform austenite) cost next to nothing, and one instance with
+// its front high up would otherwise hold the launch.  A group's size is the order of
+// its instances' sums, so the groups are sized again only for a new sweep (all
+// instances uploaded since the last run) or a new configuration: a new state for
+// some of them leaves the others their bits.  Groups asked for by name
+// (PEARL_BATCH_SIZED_GROUPS) keep the planner's sizes, and a sweep's bits hang on its
+// instances' sizes alone.  Only where the grid has two blocks an instance and fewer
+// than its tiles: below that, groups run several instances and plan_groups balances
+// them; above, every tile has a block.  96 instances of 32..192 x 64..1024 cells,
+// 20 steps: 25.7 -> 19.7 ms; 24 instances 7.7 -> 5.2.
 int batch_replan(pearl_gpu_batch* b) {
     const int max_grid = b->per_sm * b->sms;
     if (!b->replan) return PEARL_OK;
     b->replan = false;
-    if (b->group_blocks != PEARL_BATCH_SIZED_GROUPS || !b->use_tma || 2 * b->n > max_grid) return PEARL_OK;
+    if (!b->by_state || b->group_blocks != PEARL_BATCH_SIZED_GROUPS || !b->use_tma || 2 * b->n > max_grid)
+        return PEARL_OK;
     std::vector<long long> tiles(b->n);
     long long sum = 0;
     for (int i = 0; i < b->n; ++i) {
@@ -431,6 +435,7 @@ int pearl_gpu_batch_create(int n, const pearl_params* params, const int* nx, con
         cudaGetLastError();
         b->tma_capable = tma = false;
     }
+    b->by_state = group_blocks <= 0 && group_blocks != PEARL_BATCH_SIZED_GROUPS;
     const int rc = batch_configure(b, group_blocks > 0 ? group_blocks : PEARL_BATCH_SIZED_GROUPS, tma, 0);
     if (rc) return bail(rc);
     *out = b;
@@ -600,6 +605,7 @@ int pearl_gpu_batch_configure(pearl_gpu_batch* b, int group_blocks, int use_tma,
     const int wx = tile_warps_x == 1 ? 0 : tile_warps_x == 2 ? 1 : tile_warps_x == 4 ? 2 : tile_warps_x == 8 ? 3 : -1;
     if (wx < 0) return bfail(b, PEARL_ERR_INVALID_ARGUMENT, "tile_warps_x must be 1, 2, 4 or 8");
     PB_CUDA(b, cudaSetDevice(b->device));
+    b->by_state = false;
     return batch_configure(b, group_blocks, use_tma != 0, wx);
 }
 

@@ -488,6 +488,9 @@ class Batch:
 
     ``cases`` is a sequence of (params, nx, ny).  Each instance follows the
     same step path as a :class:`Context` of its own.
+    ``group_blocks``: blocks per group, BATCH_SIZED_GROUPS for groups sized by the
+    instances' tile counts, 0 for sizes that follow the uploaded states too (faster;
+    the last bits of an instance then depend on all of them, see pearl_gpu.h).
     """
 
     def __init__(self, cases, device: int = 0, group_blocks: int = 0):

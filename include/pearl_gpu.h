@@ -376,25 +376,28 @@ int pearl_gpu_adjoint_gradient(pearl_gpu_ctx* ctx, long long nsteps, int checkpo
  * the groups have per-instance sizes instead, chosen so that the slowest group
  * finishes soonest under a model of a pass's cost (powers of two up to the
  * grid, or an equal share of the grid per instance): small instances share
- * groups of a few blocks, large ones get many.  With two blocks or more
- * an instance, and fewer than one a tile, the sizes follow the uploaded states:
- * an instance gets blocks in proportion to the part of it that is not uniform
- * austenite.  They are set at the first run after all instances have been
- * uploaded with no run between, or (all of them uploaded before) after the batch
- * was configured, and kept through other runs and uploads.  The order of an instance's sums, and with it the last bits
- * of its results, depends on its group's size, here on all the states uploaded
- * for a sweep: a sweep that is downloaded and uploaded again half-way agrees with the
- * uninterrupted one to rounding.  Groups of one given size (group_blocks > 0)
- * repeat it bit for bit.  Every instance follows exactly the path of a
+ * groups of a few blocks, large ones get many.
+ * The default, group_blocks = 0, lets these sizes follow the uploaded states too,
+ * where the grid has two blocks or more an instance and fewer than one a tile: an
+ * instance gets blocks in proportion to the part of it that is not uniform
+ * austenite.  They are set at the first run after all instances have been uploaded
+ * with no run between (and after a precision change or an autotune, by the last
+ * uploads), and kept through other runs and uploads.  The order of an instance's
+ * sums, and with it the last bits of its results, depends on its group's size, then
+ * on all the states uploaded for a sweep: a sweep that is downloaded and uploaded
+ * again half-way agrees with the uninterrupted one to rounding.  With
+ * PEARL_BATCH_SIZED_GROUPS by name the sizes depend on the instances' tile counts
+ * alone, and such a sweep repeats the uninterrupted one bit for bit, as it does with
+ * groups of one given size.  Every instance follows exactly the path of a
  * pearl_gpu_ctx (same kernels, same reduction order for the same group size),
  * so it is main's loop (pearl_serial.cpp:2296-2306) run once per instance.
  * No counterpart in the reference, which runs one case per process. */
 typedef struct pearl_gpu_batch pearl_gpu_batch;
 enum { PEARL_BATCH_SIZED_GROUPS = -1 };
 
-/* group_blocks: blocks per group, or any value <= 0 (PEARL_BATCH_SIZED_GROUPS
- * among them) for groups sized per instance; pearl_gpu_batch_autotune can
- * choose instead. */
+/* group_blocks: blocks per group, PEARL_BATCH_SIZED_GROUPS for groups sized per
+ * instance, or 0 (or any value below -1) for such groups that follow the uploaded
+ * states too; pearl_gpu_batch_autotune can choose instead. */
 int pearl_gpu_batch_create(int n, const pearl_params* params, const int* nx, const int* ny, int device,
                            int group_blocks, pearl_gpu_batch** out);
 void pearl_gpu_batch_destroy(pearl_gpu_batch* batch);
@@ -421,7 +424,7 @@ int pearl_gpu_batch_autotune(pearl_gpu_batch* batch, int steps, int* group_block
 /* pearl_gpu_set_precision for every instance. */
 int pearl_gpu_batch_set_precision(pearl_gpu_batch* batch, int precision);
 /* Sets the configuration pearl_gpu_batch_autotune would choose: blocks per
- * group (or PEARL_BATCH_SIZED_GROUPS, with the fixed-cost weight the last
+ * group (or PEARL_BATCH_SIZED_GROUPS: by tile counts alone, with the fixed-cost weight the last
  * autotune chose, initially 4 tiles), TMA staging (used only with
  * tile_warps_x = 1) and the tile shape (tile_warps_x warps side by side in x:
  * 1, 2, 4 or 8). */

@@ -141,3 +141,30 @@ def test_autotune_leaves_the_groups_that_run(gpu_lib):
         timed = b.stats()["grid"]
         _run(b, 2)
         assert timed == b.stats()["grid"] == sum(sizes)
+
+
+def test_groups_sized_by_tiles_alone_repeat_a_sweep(gpu_lib, port):
+    """PEARL_BATCH_SIZED_GROUPS asked for by name: sizes follow the instances' tile
+    counts, and a sweep that is downloaded and uploaded again half-way, after the
+    fronts have been made to look elsewhere, repeats the uninterrupted one bit for bit."""
+    import pearl_gpu
+
+    ws = _workloads(LOW)
+    _, sizes, _ = pearl_gpu.batch_plan([-(-nx // 32) * -(-ny // 16) for nx, ny in SIZES], GRID,
+                                       pearl_gpu.BATCH_SIZED_GROUPS)
+    assert len(sizes) == 3 and list(sizes) != _groups(ws)
+    cases = [(w.params, w.nx, w.ny) for w in ws]
+    with pearl_gpu.Batch(cases, group_blocks=pearl_gpu.BATCH_SIZED_GROUPS) as b, pearl_gpu.Batch(cases) as c:
+        c.configure(pearl_gpu.BATCH_SIZED_GROUPS)
+        for batch in (b, c):
+            _upload(batch, ws)
+            _run(batch, 2)
+            half = [batch.download(i) for i in range(3)]
+            _upload(batch, _workloads(HIGH))
+            _run(batch, 1)
+            for i, state in enumerate(half):
+                batch.upload(i, *state)
+            reports = _run(batch, 2)
+            assert batch.stats()["grid"] == sum(sizes)
+            for i, w in enumerate(ws):
+                _check(port, batch, reports, i, w, int(sizes[i]), 4)
